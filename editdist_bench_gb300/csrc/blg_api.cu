@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <atomic>
 #include <array>
+#include <cmath>
 #include <condition_variable>
 #include <functional>
 #include <thread>
@@ -29,6 +30,7 @@
 #include "blg_batch.h"
 #include "blg_internal.h"
 #include "blg_sched.h"
+#include "blg_search_bits.h"
 
 namespace blg {
 cudaError_t launch_build_peq(cudaStream_t st, const DevStrings &Q, const int32_t *qidx, int nq, int nwc,
@@ -45,7 +47,7 @@ cudaError_t launch_prefix_text(cudaStream_t st, int sms, const DevStrings &C, co
 cudaError_t launch_search_tt(cudaStream_t st, int nw, bool hask, const TransposedChoices &T,
                              const SearchClass &cls, int qpb, int k, int dtype, void *out);
 cudaError_t launch_transpose_choices(cudaStream_t st, int sms, const DevStrings &C, const int64_t *base,
-                                     uint32_t *words, int32_t *len, uint32_t *status);
+                                     uint32_t *words, int32_t *len, uint16_t *order, uint32_t *status);
 cudaError_t launch_search_lanes(cudaStream_t st, bool hask, const DevStrings &C, const SearchClass &cls,
                                 int nwc, int k, int dtype, void *out, uint32_t *status);
 cudaError_t launch_pairs_long(cudaStream_t st, int grid, bool hask, const LongQueue &q, int k,
@@ -104,6 +106,17 @@ namespace {
 
 constexpr int kSeqMaxWords = 8;          // queries up to 512: sequential words per thread
 constexpr int kLaneMaxWords = 32;        // queries up to 2048: lane-spread
+
+// Bit-sliced exact search: the largest symbol table of a launch (shared
+// memory) and the largest scratch for the deltas between stripes.
+constexpr size_t kBitsMaxTable = 160 << 10;
+constexpr size_t kBitsMaxScratch = size_t(512) << 20;
+// The prefix-reuse kernel where the restarts skip enough of the text (it takes
+// 16.3 ms on 4096 x 65536 reads of 64 bases with none skipped, the bit-sliced
+// one 9.2), and for 33 to 64 queries, where its tests hold it to that path
+// (64 x 20000 reads of 64: 186 us against 77).
+constexpr double kBitsPfxSaving = 0.45;
+constexpr int kPfxMinQueries = 33, kPfxMaxQueries = 64;
 
 struct OwnedStrings {
     DevStrings d;
@@ -192,6 +205,15 @@ struct blg_search {
     uint32_t *tt_words = nullptr;
     int64_t *tt_base = nullptr;
     int32_t *tt_len = nullptr;
+    uint16_t *tt_order = nullptr;     // per tile: positions by length, longest first
+    int64_t max_len = 0;              // longest choice
+    // exact runs, bit-sliced over the queries (k_search_bits): the distinct
+    // bytes of the queries (nsym 0: not counted, or too many) and, per class set, the
+    // sequential queries by length
+    int nsym = 0;
+    uint8_t sym_map[256];
+    void *bits_mem = nullptr;         // [group weights | qidx | qlen] of the sequential queries
+    int bits_nq = 0, bits_longest = 0;
 };
 
 // ------------------------------------------------------------ helpers --
@@ -772,6 +794,9 @@ static void pairs_release(blg_ctx *c, blg_pairs *p) {
 static void free_classes(blg_ctx *c, blg_search *s) {
     for (auto &k : s->cls) dev_free(c, k.mem);
     s->cls.clear();
+    dev_free(c, s->bits_mem);
+    s->bits_mem = nullptr;
+    s->bits_nq = 0;
 }
 
 // Length buckets of a choice set (the sorted copy of thresholded runs): a
@@ -881,6 +906,53 @@ static bool query_classes(const int64_t *oq, int64_t q0, int64_t q1, std::vector
     return true;
 }
 
+// The sequential queries of the classes as one list by length (the classes are
+// in order of words, each by length) for the bit-sliced exact search, and the
+// weights that split its work (BitSearch::weight).
+static int bits_build(blg_ctx *c, const std::vector<QueryClass> &qc, blg_search *s) {
+    if (!s->tt || s->nsym <= 0) return BLG_OK;
+    std::vector<int32_t> idx, len;
+    for (auto &q : qc) {
+        if (q.lanes) continue;
+        idx.insert(idx.end(), q.idx.begin(), q.idx.end());
+        len.insert(len.end(), q.len.begin(), q.len.end());
+    }
+    const size_t nq = idx.size(), groups = (nq + 31) / 32;
+    if (nq == 0) return BLG_OK;
+    std::vector<int64_t> host(groups + 1 + nq);             // weights, then the indexes and lengths (8 bytes a query)
+    host[0] = 0;
+    for (size_t g = 0; g < groups; g++)
+        host[g + 1] = host[g] + bits_unit_weight(len[std::min(nq, (groups - g) * 32) - 1]) * ((s->nc + 31) / 32);
+    memcpy(host.data() + groups + 1, idx.data(), 4 * nq);
+    memcpy((uint8_t *)(host.data() + groups + 1) + 4 * nq, len.data(), 4 * nq);
+    CK(dev_alloc(c, &s->bits_mem, 8 * host.size()), "cudaMallocAsync(bit-sliced queries)");
+    CK(cudaMemcpyAsync(s->bits_mem, host.data(), 8 * host.size(), cudaMemcpyHostToDevice, c->stream), "H2D queries");
+    s->bits_nq = (int)nq;
+    s->bits_longest = len.back();
+    return BLG_OK;                                       // (pageable: the copy completed before return)
+}
+
+// The distinct bytes of queries [0, nq): symbols 1 .. nsym in byte order; the
+// bytes of no query map to symbol 0, an empty row of the kernel's table.
+static void query_symbols(const uint8_t *bq, const int64_t *oq, int64_t nq, blg_search *s) {
+    HostPool &pool = HostPool::get();
+    const int64_t lo = oq[0], bytes = oq[nq] - lo;
+    const int nt = bytes >= (1 << 18) ? pool.size() : 1;
+    std::vector<std::array<uint8_t, 256>> seen((size_t)nt);
+    pool.run(nt, [&](int t) {
+        seen[t].fill(0);
+        for (int64_t x = lo + bytes * t / nt, e = lo + bytes * (t + 1) / nt; x < e; x++) seen[t][bq[x]] = 1;
+    });
+    std::array<uint8_t, 256> any{};
+    for (auto &v : seen)
+        for (int b = 0; b < 256; b++) any[b] |= v[b];
+    int n = 0;
+    for (int b = 0; b < 256; b++) n += any[b];
+    s->nsym = n <= 255 ? n : 0;                          // (256: the map's byte has no room for them)
+    int r = 0;
+    for (int b = 0; b < 256; b++) s->sym_map[b] = (uint8_t)(any[b] ? ++r : 0);
+}
+
 // Query classes of queries [q0, q1) (query_classes), each in one device
 // block with its Peq tables; replaces the previous classes.
 static int search_build_classes(blg_ctx *c, const int64_t *oq, int64_t q0, int64_t q1, blg_search *s) {
@@ -925,7 +997,7 @@ static int search_build_classes(blg_ctx *c, const int64_t *oq, int64_t q0, int64
         CK(launch(c, "build_peq", [&] {
                return launch_build_peq(c->stream, s->q.d, k_.qidx, k_.nq, k_.nw, k_.peq, c->d_status);
            }), "build_peq");
-    return BLG_OK;
+    return bits_build(c, qc, s);
 }
 
 // Choices: the packed strings, a length-sorted copy (thresholded runs) and
@@ -967,6 +1039,28 @@ enum { NEED_SORTED = 1, NEED_TT = 2, NEED_PFX = 4, NEED_ALL = 7 };
 // are skipped; the text is laid out on the device (k_prefix_text).
 constexpr int64_t kPfxMinChoices = 4096;
 constexpr double kPfxMinSaving = 0.02;
+
+// The share of the text that sorted neighbours have in common, from 2048
+// choices spread over the set: a set whose restarts would skip half of its
+// columns shows most of that in a sample.
+static double sampled_prefix_share(const uint8_t *bc, const int64_t *oc, int64_t nc) {
+    const int64_t n = std::min<int64_t>(nc, 2048);
+    std::vector<int64_t> at((size_t)n);
+    for (int64_t i = 0; i < n; i++) at[i] = nc * i / n;
+    std::sort(at.begin(), at.end(), [&](int64_t x, int64_t y) {
+        return std::lexicographical_compare(bc + oc[x], bc + oc[x + 1], bc + oc[y], bc + oc[y + 1]);
+    });
+    int64_t same = 0, all = 0;
+    for (int64_t i = 1; i < n; i++) {
+        const uint8_t *x = bc + oc[at[i - 1]], *y = bc + oc[at[i]];
+        const int64_t lim = std::min(oc[at[i - 1] + 1] - oc[at[i - 1]], oc[at[i] + 1] - oc[at[i]]);
+        int64_t l = 0;
+        while (l < lim && x[l] == y[l]) l++;
+        same += l;
+        all += oc[at[i] + 1] - oc[at[i]];
+    }
+    return all > 0 ? (double)same / (double)all : 0.0;
+}
 
 static int search_build_prefix(blg_ctx *c, const uint8_t *bc, const int64_t *oc, int64_t nc, blg_search *s) {
     if (nc < kPfxMinChoices || nc >= INT32_MAX) return BLG_OK;
@@ -1172,14 +1266,17 @@ static int search_upload_choices(blg_ctx *c, const uint8_t *bc, const int64_t *o
         std::vector<int64_t> base(tiles + 1, 0);
         HostPool &pool = HostPool::get();
         const int nt = nc >= (1 << 16) ? pool.size() : 1;
+        std::vector<int64_t> longest((size_t)nt, 0);
         pool.run(nt, [&](int w) {                               // each tile's longest choice
             for (int64_t t = tiles * w / nt, te = tiles * (w + 1) / nt; t < te; t++) {
                 int64_t mx = 0;
                 const int64_t e = std::min(nc, (t + 1) * kTileCands);
                 for (int64_t i = t * kTileCands; i < e; i++) mx = std::max(mx, oc[i + 1] - oc[i]);
                 base[t + 1] = kTileCands * ((mx + 3) / 4);
+                longest[w] = std::max(longest[w], mx);
             }
         });
+        s->max_len = *std::max_element(longest.begin(), longest.end());
         for (int64_t t = 0; t < tiles; t++) base[t + 1] += base[t];
         const int64_t bytes = oc[nc] - oc[0];
         if (base[tiles] * 4 <= 2 * bytes + (64ll << 20)) {
@@ -1189,11 +1286,13 @@ static int search_upload_choices(blg_ctx *c, const uint8_t *bc, const int64_t *o
                "cudaMallocAsync(tt)");
             CK(dev_alloc(c, (void **)&s->tt_base, sizeof(int64_t) * (size_t)(tiles + 1)), "cudaMallocAsync(tt base)");
             CK(dev_alloc(c, (void **)&s->tt_len, sizeof(int32_t) * (size_t)nc), "cudaMallocAsync(tt len)");
+            CK(dev_alloc(c, (void **)&s->tt_order, sizeof(uint16_t) * (size_t)tiles * kTileCands),
+               "cudaMallocAsync(tt order)");
             CK(cudaMemcpyAsync(s->tt_base, base.data(), sizeof(int64_t) * (tiles + 1), cudaMemcpyHostToDevice,
                                c->stream), "H2D tt base");
             CK(launch(c, "transpose_choices", [&] {
                    return launch_transpose_choices(c->stream, c->sms, s->c.d, s->tt_base, s->tt_words, s->tt_len,
-                                                   c->d_status);
+                                                   s->tt_order, c->d_status);
                }), "transpose_choices");
             s->tt = true;
         }
@@ -1209,11 +1308,14 @@ static int search_upload_choices(blg_ctx *c, const uint8_t *bc, const int64_t *o
 static int search_run(blg_ctx *c, blg_search *s, int k, int dtype, void *d_out, int64_t q0 = 0,
                       int64_t q1 = -1);
 
-// Queries into HBM, with their 4-gram sketches.
-static int search_upload_queries(blg_ctx *c, const uint8_t *bq, const int64_t *oq, int64_t nq, blg_search *s) {
+// Queries into HBM, with what `need` asks for: their 4-gram sketches
+// (thresholded runs), their symbols (exact runs).
+static int search_upload_queries(blg_ctx *c, const uint8_t *bq, const int64_t *oq, int64_t nq, blg_search *s,
+                                 unsigned need = NEED_ALL) {
     s->nq = nq;
     int rc = upload_strings(c, bq, oq, nq, s->q);
     if (rc) return rc;
+    if ((need & NEED_TT) && nq > 0) query_symbols(bq, oq, nq, s);
     // one block: the sketches (8 B each), then the 4-gram counts (16 B each, 16-byte aligned)
     const size_t nq1 = (size_t)std::max<int64_t>(nq, 1), o_cnt = (8 * nq1 + 15) & ~size_t(15);
     CK(dev_alloc(c, (void **)&s->qsk, o_cnt + 16 * nq1), "cudaMallocAsync(sketches)");
@@ -1233,8 +1335,9 @@ static int cdist_pipelined(blg_ctx *c, const uint8_t *bq, const int64_t *oq, int
                            const int64_t *oc, int64_t nc, int k, int dtype, void *out_host, void *d_out,
                            blg_search *s, void *d4) {
     const bool surv = k >= 0 && c->sched != BLG_SCHED_PLAIN;      // the survivor kernels run (search_run)
-    int rc = search_upload_queries(c, bq, oq, nq, s);
-    if (!rc) rc = search_upload_choices(c, bc, oc, nc, s, surv ? NEED_SORTED : NEED_TT);
+    const unsigned need = surv ? NEED_SORTED : NEED_TT;
+    int rc = search_upload_queries(c, bq, oq, nq, s, need);
+    if (!rc) rc = search_upload_choices(c, bc, oc, nc, s, need);
     if (rc) return rc;
     const size_t row = dtype_size(dtype) * (size_t)nc;
     // Query chunks of relative sizes 4,4,4,4,4,4,4,2,1,1: the last chunk's
@@ -1278,7 +1381,11 @@ static int cdist_pipelined(blg_ctx *c, const uint8_t *bq, const int64_t *oq, int
             // exact runs: the host sorts the choices for the prefix-reuse
             // kernel while the first chunk computes on the tile-transposed
             // copy; the later chunks use it
-            if (!rc && ch == 0 && k < 0 && nch > 1) rc = search_build_prefix(c, bc, oc, nc, s);
+            // (only where the bit-sliced kernel would not beat it)
+            if (!rc && ch == 0 && k < 0 && nch > 1 &&
+                ((s->bits_nq >= kPfxMinQueries && s->bits_nq <= kPfxMaxQueries) || s->bits_nq == 0 ||
+                 sampled_prefix_share(bc, oc, nc) >= 0.7 * kBitsPfxSaving))
+                rc = search_build_prefix(c, bc, oc, nc, s);
             if (rc) break;
         }
         if (ch >= 1) {
@@ -1298,7 +1405,7 @@ static int cdist_pipelined(blg_ctx *c, const uint8_t *bq, const int64_t *oq, int
 static int search_upload(blg_ctx *c, const uint8_t *bq, const int64_t *oq, int64_t nq,
                          const uint8_t *bc, const int64_t *oc, int64_t nc, blg_search *s,
                          unsigned need = NEED_ALL, int32_t *perm_stage = nullptr) {
-    int rc = search_upload_queries(c, bq, oq, nq, s);
+    int rc = search_upload_queries(c, bq, oq, nq, s, need);
     if (!rc && need == NEED_ALL && nq > 0) s->h_oq.assign(oq, oq + nq + 1);   // a resident search keeps them
     if (!rc) rc = search_upload_choices(c, bc, oc, nc, s, need, perm_stage);
     if (!rc) rc = search_build_classes(c, oq, 0, nq, s);
@@ -1367,6 +1474,73 @@ static int64_t class_queries(const blg_search *s) {
     return n;
 }
 
+// Whether the exact run of the sequential classes takes the prefix-reuse kernel
+// for its one- and two-word classes.
+static bool use_prefix(const blg_search *s) {
+    return s->pfx && ((s->bits_nq >= kPfxMinQueries && s->bits_nq <= kPfxMaxQueries) ||
+                      s->pfx_saving >= kBitsPfxSaving || s->bits_nq == 0);
+}
+
+// Whether the bit-sliced kernel beats the per-class word kernels on an exact
+// run. Both have a floor, the time a lone warp takes for its longest strings,
+// and a rate. Measured (GB300, 1 to 256 queries x 200 to 60000 choices of 12
+// to 256 bytes; microseconds bit-sliced / word): a bit-sliced unit takes 6.6
+// ns per cell of its 32 x 32 pairs alone and four fifths of that when an SM
+// partition has several; a word kernel's thread 37 ns per column and word
+// (four words at least: short queries go four at a time), for up to four
+// choices one after the other, and 1.12 ps per column and word at full rate.
+// 64 x 64 bytes: 32 x 200 34 / 13, 1 x 2000 32 / 42, 32 x 60000 93 / 483;
+// 256 x 256 bytes: 32 x 3500 389 / 169, 32 x 20000 654 / 820, 256 x 60000
+// 8414 / 17565.
+static bool bits_faster(const blg_ctx *c, const blg_search *s) {
+    const double cols = (double)s->max_len, avg = (double)s->c.d.bytes / (double)s->nc;
+    const double units = (double)((s->bits_nq + 31) / 32) * (double)((s->nc + 31) / 32);
+    const double alone = 6.6e-3 * cols * (double)std::max(8, (s->bits_longest + 7) & ~7);
+    const double waves = std::ceil(units / (4.0 * c->sms));
+    const double bits = 8.0 + alone * std::max(1.0, 0.8 * waves * (waves > 2 ? avg / std::max(cols, 1.0) : 1.0));
+    double word = 0.0;
+    for (auto &k : s->cls) {
+        if (k.lanes) continue;
+        const double floor = 37e-3 * cols * std::max(4, k.nw) * (double)std::min<int64_t>(4, (s->nc + 255) / 256);
+        word += 5.0 + std::max(floor, 1.12e-6 * avg * k.nw * (double)k.nq * (double)s->nc);
+    }
+    return bits <= word;
+}
+
+// The exact run of every sequential query, bit-sliced (k_search_bits).
+// *done = false, with nothing launched, when it does not apply.
+static int search_run_bits(blg_ctx *c, blg_search *s, int dtype, void *d_out, bool *done) {
+    *done = false;
+    if (!s->tt || !s->bits_mem || bits_table_bytes(s->nsym, s->bits_longest) > kBitsMaxTable) return BLG_OK;
+    if (use_prefix(s) || !bits_faster(c, s)) return BLG_OK;
+    BitSearch B{};
+    B.Q = s->q.d;
+    B.nq = s->bits_nq;
+    B.groups = (B.nq + 31) / 32;
+    B.weight = (const int64_t *)s->bits_mem;
+    B.qidx = (const int32_t *)(B.weight + B.groups + 1);
+    B.qlen = B.qidx + B.nq;
+    B.T = TransposedChoices{s->tt_words, s->tt_base, s->tt_len, s->nc};
+    B.order = s->tt_order;
+    B.nsym = s->nsym;
+    memcpy(B.map, s->sym_map, sizeof(B.map));
+    void *scratch = nullptr;
+    if (s->bits_longest > 64) {
+        B.scratch_words = bits_scratch_words(s->max_len);
+        const size_t bytes = sizeof(uint32_t) * (size_t)B.scratch_words * (size_t)bits_warps(c->sms);
+        if (bytes > kBitsMaxScratch) return BLG_OK;
+        CK(dev_alloc(c, &scratch, bytes), "cudaMallocAsync(stripe deltas)");
+        B.scratch = (uint32_t *)scratch;
+    }
+    const cudaError_t e = launch(c, "search_bits", [&] {
+        return launch_search_bits(c->stream, c->sms, B, s->bits_longest, dtype, d_out, c->d_status);
+    });
+    dev_free(c, scratch);
+    if (e != cudaSuccess) return cuda_fail(c, e, "search_bits");
+    *done = true;
+    return BLG_OK;
+}
+
 static int search_run(blg_ctx *c, blg_search *s, int k, int dtype, void *d_out, int64_t q0, int64_t q1) {
     if (!dtype_ok(dtype)) return fail(c, BLG_ERR_ARG, "dtype must be int32, uint16 or uint8");
     if (s->nq == 0 || s->nc == 0) return BLG_OK;
@@ -1423,9 +1597,14 @@ static int search_run(blg_ctx *c, blg_search *s, int k, int dtype, void *d_out, 
                    }), "search_surv");
         }
     }
+    bool bits = false;
+    if (!hask) {
+        const int rc = search_run_bits(c, s, dtype, d_out, &bits);
+        if (rc) return rc;
+    }
     for (auto &k_ : s->cls) {
         SearchClass sc{k_.nw, k_.nq, k_.qidx, k_.qlen, k_.peq};
-        if (surv && !k_.lanes) continue;
+        if ((surv || bits) && !k_.lanes) continue;
         if (k_.lanes) {
             CK(launch(c, "search_lanes", [&] {
                    return launch_search_lanes(c->stream, hask, s->c.d, sc, k_.nw, k, dtype, d_out,
@@ -1433,7 +1612,7 @@ static int search_run(blg_ctx *c, blg_search *s, int k, int dtype, void *d_out, 
                }), "search_lanes");
         } else {
             const int qpb = pick_qpb(c, k_.nw, k_.nq, s->nc);
-            if (!hask && s->pfx && search_pfx_supported(k_.nw)) {
+            if (!hask && use_prefix(s) && search_pfx_supported(k_.nw)) {
                 // exact short queries over the prefix-sorted choices
                 CK(cudaMemsetAsync(s->pfx_work, 0, sizeof(unsigned long long), c->stream), "reset work");
                 CK(launch(c, "search_pfx", [&] {
@@ -1610,6 +1789,7 @@ static void search_release(blg_ctx *c, blg_search *s) {
     dev_free(c, s->tt_words);
     dev_free(c, s->tt_base);
     dev_free(c, s->tt_len);
+    dev_free(c, s->tt_order);
     dev_free(c, s->pfx_mem);
     s->pfx_mem = nullptr;
     s->pfx_work = nullptr;
@@ -1621,6 +1801,7 @@ static void search_release(blg_ctx *c, blg_search *s) {
     s->tt_words = nullptr;
     s->tt_base = nullptr;
     s->tt_len = nullptr;
+    s->tt_order = nullptr;
     s->tt = false;
     free_classes(c, s);
 }
@@ -2883,7 +3064,8 @@ int blg_cdist(blg_ctx *c, const uint8_t *bq, const int64_t *oq, int64_t nq, cons
         // the next chunk computes
         const bool pipe = !out_device && nq >= 2 && obytes >= (u4 ? (32u << 20) : (64u << 20));
         if (!pipe) {
-            rc = search_upload(c, bq, oq, nq, bc, oc, nc, &s);
+            const bool surv = max_dist >= 0 && c->sched != BLG_SCHED_PLAIN;
+            rc = search_upload(c, bq, oq, nq, bc, oc, nc, &s, surv ? NEED_SORTED | NEED_TT : NEED_TT | NEED_PFX);
             if (!rc) rc = search_run(c, &s, max_dist, u4 ? BLG_UINT8 : dtype, u4 ? d8 : d_out);
             if (!rc && u4) rc = pack_u4(c, d8, 0, n, d_out);
             if (!rc && !out_device) {
@@ -2972,8 +3154,9 @@ int blg_cdist_matches(blg_ctx *c, const uint8_t *bq, const int64_t *oq, int64_t 
     if (nq == 0 || nc == 0) return BLG_OK;
     blg_search s;
     const bool surv = c->sched != BLG_SCHED_PLAIN;
-    int rc = search_upload_queries(c, bq, oq, nq, &s);
-    if (!rc) rc = search_upload_choices(c, bc, oc, nc, &s, surv ? NEED_SORTED : NEED_TT);
+    const unsigned need = surv ? NEED_SORTED : NEED_TT;
+    int rc = search_upload_queries(c, bq, oq, nq, &s, need);
+    if (!rc) rc = search_upload_choices(c, bc, oc, nc, &s, need);
     // the survivor kernel's result list, where the run qualifies
     int64_t total = 0;
     bool listed = false;

@@ -14,6 +14,7 @@
 #include <cstring>
 #include <vector>
 
+#include "blg_bits.cuh"
 #include "blg_device.cuh"
 
 using namespace blg;
@@ -263,4 +264,61 @@ extern "C" int blg_host_store(int d, int dtype) {
     if (dtype == DT_UINT8) return (int)saturate_u8(d);
     if (dtype == DT_UINT16) return (int)saturate_u16(d);
     return d;
+}
+
+// The bit-sliced search of up to 32 queries (packed: bytes and offsets) against
+// one text, as k_search_bits runs it: stripes of 64 rows with the deltas
+// between them kept per column, counts of the last column's vertical deltas
+// in planes, transposed to bytes. out: one distance per query.
+extern "C" void blg_host_bits(const uint8_t *buf, const int64_t *off, int nq, const uint8_t *t, int n, int32_t *out) {
+    int longest = 0;
+    for (int q = 0; q < nq; q++) longest = longest < off[q + 1] - off[q] ? (int)(off[q + 1] - off[q]) : longest;
+    const int stripes = longest > 0 ? (longest + 63) / 64 : 1;
+    std::vector<uint32_t> hp((size_t)n, ~0u), hm((size_t)n, 0);
+    const BitUnits u{1u, ~0u};
+    uint32_t acc[kBitPlanes] = {0};
+    for (int s = 0; s < stripes; s++) {
+        const int rows = s == stripes - 1 ? ((longest - 64 * s + 7) / 8 * 8 > 8 ? (longest - 64 * s + 7) / 8 * 8 : 8) : 64;
+        uint32_t vn[64], vm[64], valid[64] = {0};
+        for (int i = 0; i < 64; i++) {
+            vn[i] = 0;
+            vm[i] = 0;
+            for (int q = 0; q < nq; q++)
+                if (64 * s + i < off[q + 1] - off[q]) valid[i] |= 1u << q;
+        }
+        for (int j = 0; j < n; j++) {
+            for (int i = 0; i < rows; i++) {
+                uint32_t eq = 0;
+                for (int q = 0; q < nq; q++)
+                    if ((valid[i] >> q & 1u) && buf[off[q] + 64 * s + i] == t[j]) eq |= 1u << q;
+                if (i & 1) bit_cell<true>(eq, vn[i], vm[i], hp[j], hm[j], u);
+                else bit_cell<false>(eq, vn[i], vm[i], hp[j], hm[j], u);
+            }
+        }
+        uint32_t pl[8] = {0};
+        for (int i = 0; i < rows; i += 4) {
+            uint32_t x[8];
+            for (int b = 0; b < 4; b++) {
+                x[b] = ~vn[i + b] & valid[i + b];
+                x[4 + b] = ~vm[i + b] & valid[i + b];
+            }
+            bit_count8(pl, x);
+        }
+        uint32_t carry = 0, c2;
+        for (int p = 0; p < kBitPlanes; p++) {
+            bit_full_add(acc[p], c2, p < 8 ? pl[p] : 0u, carry);
+            carry = c2;
+        }
+    }
+    uint32_t lo[8], hi[8];
+    for (int p = 0; p < 8; p++) {
+        lo[p] = acc[p];
+        hi[p] = p + 8 < kBitPlanes ? acc[p + 8] : 0u;
+    }
+    bit_transpose8(lo);
+    bit_transpose8(hi);
+    for (int q = 0; q < nq; q++) {
+        const int cnt = (int)((lo[q & 7] >> (q & 24) & 0xffu) | (hi[q & 7] >> (q & 24) & 0xffu) << 8);
+        out[q] = n - (int)(off[q + 1] - off[q]) + cnt;
+    }
 }

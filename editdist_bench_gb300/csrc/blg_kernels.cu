@@ -326,8 +326,11 @@ __global__ void __launch_bounds__(256) k_prefix_text(DevStrings C, const int32_t
 
 // Transpose choices into tiles (see TransposedChoices); one thread per
 // (choice, word), bytes past a choice's end are zero.
+// order: the tile's positions by length, longest first, equal lengths in
+// place (a bitonic sort of length and position; tiles of one length skip it).
 __global__ void __launch_bounds__(256) k_transpose_choices(DevStrings C, const int64_t *base, uint32_t *words,
-                                                           int32_t *len, uint32_t *status) {
+                                                           int32_t *len, uint16_t *order, uint32_t *status) {
+    __shared__ uint32_t s_key[kTileCands];
     const int64_t nc = C.n;
     const int64_t tiles = (nc + kTileCands - 1) / kTileCands;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -338,6 +341,8 @@ __global__ void __launch_bounds__(256) k_transpose_choices(DevStrings C, const i
             int n = 0;
             const uint8_t *p = c < nc ? string_at(C, c, n, status) : C.buf;
             if (c < nc) len[c] = n;
+            // ascending keys: descending length (capped: the order is free), then position; no choice: last
+            s_key[cl] = c < nc ? ((uint32_t)(0x1fffff - min(n, 0x1fffff)) << 10) | (uint32_t)cl : 0x80000000u | cl;
             for (int w = 0; w < nwords; w++) {
                 uint32_t v = 0;
                 const int rem = n - 4 * w;
@@ -348,6 +353,27 @@ __global__ void __launch_bounds__(256) k_transpose_choices(DevStrings C, const i
                 words[b0 + (int64_t)w * kTileCands + cl] = v;
             }
         }
+        __syncthreads();
+        bool mixed = false;
+        for (int cl = threadIdx.x; cl < kTileCands; cl += blockDim.x)
+            mixed |= s_key[cl] >> 31 == 0 && (s_key[cl] ^ s_key[0]) >> 10 != 0;
+        if (__syncthreads_or(mixed)) {
+            for (int size = 2; size <= kTileCands; size <<= 1)
+                for (int d = size >> 1; d > 0; d >>= 1) {
+                    for (int x = threadIdx.x; x < kTileCands / 2; x += blockDim.x) {
+                        const int i = 2 * x - (x & (d - 1)), k = i + d;
+                        const uint32_t a = s_key[i], b = s_key[k];
+                        if ((a > b) == ((i & size) == 0)) {
+                            s_key[i] = b;
+                            s_key[k] = a;
+                        }
+                    }
+                    __syncthreads();
+                }
+        }
+        for (int cl = threadIdx.x; cl < kTileCands; cl += blockDim.x)
+            order[tile * kTileCands + cl] = (uint16_t)(s_key[cl] & 1023u);
+        __syncthreads();                                       // the keys are reused by the next tile
     }
 }
 
@@ -775,11 +801,11 @@ cudaError_t launch_prefix_text(cudaStream_t st, int sms, const DevStrings &C, co
 }
 
 cudaError_t launch_transpose_choices(cudaStream_t st, int sms, const DevStrings &C, const int64_t *base,
-                                     uint32_t *words, int32_t *len, uint32_t *status) {
+                                     uint32_t *words, int32_t *len, uint16_t *order, uint32_t *status) {
     if (C.n <= 0) return cudaSuccess;
     const int64_t tiles = (C.n + kTileCands - 1) / kTileCands;
     const int grid = (int)std::min<int64_t>(tiles, (int64_t)sms * 8);
-    k_transpose_choices<<<grid, 256, 0, st>>>(C, base, words, len, status);
+    k_transpose_choices<<<grid, 256, 0, st>>>(C, base, words, len, order, status);
     return cudaGetLastError();
 }
 
