@@ -23,9 +23,10 @@ HOSTCHECK = os.path.join(HERE, "libblg_hostcheck.so")
 PROBE = os.path.join(HERE, "libblg_probe.so")
 
 CU_SOURCES = ["blg_api.cu", "blg_kernels.cu", "blg_noalloc.cu", "blg_pairs_sched.cu", "blg_mlp.cu", "blg_batch.cu",
-              "blg_pairs_tile.cu", "blg_search_band.cu", "blg_search_bits.cu", "blg_matches.cu"]
+              "blg_pairs_tile.cu", "blg_search_band.cu", "blg_search_bits.cu",
+              "blg_search_filter.cu", "blg_matches.cu"]
 HEADERS = ["blg_device.cuh", "blg_internal.h", "blg_kernels.cuh", "blg_context.h", "blg_sched.h", "blg_batch.h", "blg_tma.cuh",
-           "blg_bits.cuh", "blg_search_bits.h"]
+           "blg_bits.cuh", "blg_search_bits.h", "blg_search_filter.h", "blg_sig.cuh"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 
@@ -122,7 +123,7 @@ def build_packer(force: bool = False) -> str | None:
 def build_hostcheck(force: bool = False) -> str:
     """g++ build of the device header's host path (blg_hostcheck.cpp)."""
     src = os.path.join(CSRC, "blg_hostcheck.cpp")
-    deps = [src, os.path.join(CSRC, "blg_device.cuh"), os.path.join(CSRC, "blg_bits.cuh")]
+    deps = [src, os.path.join(CSRC, "blg_device.cuh"), os.path.join(CSRC, "blg_bits.cuh"), os.path.join(CSRC, "blg_sig.cuh")]
     if (not force and os.path.exists(HOSTCHECK)
             and os.path.getmtime(HOSTCHECK) >= max(os.path.getmtime(d) for d in deps)):
         return HOSTCHECK

@@ -31,6 +31,8 @@
 #include "blg_internal.h"
 #include "blg_sched.h"
 #include "blg_search_bits.h"
+#include "blg_search_filter.h"
+#include "blg_sig.cuh"
 
 namespace blg {
 cudaError_t launch_build_peq(cudaStream_t st, const DevStrings &Q, const int32_t *qidx, int nq, int nwc,
@@ -84,9 +86,8 @@ bool sched_model_trained(const blg_sched_model *m);
 namespace blg {
 cudaError_t launch_sorted_offsets(cudaStream_t st, int sms, const int64_t *lstart, int64_t n_len, int64_t min_len,
                                   const int64_t *bstart, int64_t n, int64_t *soff);
-cudaError_t launch_gather_strings(cudaStream_t st, int sms, const DevStrings &src, const int32_t *perm,
-                                  const int64_t *dst_off, uint8_t *dst, int64_t n, uint32_t *status);
-cudaError_t launch_sketch_strings(cudaStream_t st, int sms, const DevStrings &S, uint64_t *sketch, uint4 *counts,
+cudaError_t launch_sketch_strings(cudaStream_t st, int sms, const DevStrings &S, const int32_t *perm,
+                                  const int64_t *dst_off, uint8_t *dst, uint32_t *sig, uint4 *counts,
                                   uint32_t *status);
 cudaError_t launch_search_band(cudaStream_t st, int sms, int ctas_per_sm, int round, int jobsz, const SurvClasses &C,
                                const DevStrings &CS, const int32_t *perm, const uint4 *ccnt, const uint4 *qcnt, int k,
@@ -117,6 +118,8 @@ constexpr size_t kBitsMaxScratch = size_t(512) << 20;
 // (64 x 20000 reads of 64: 186 us against 77).
 constexpr double kBitsPfxSaving = 0.45;
 constexpr int kPfxMinQueries = 33, kPfxMaxQueries = 64;
+// Tensor-core filter: pairs below which its launch costs more than it saves.
+constexpr double kFltMinPairs = 1e6;
 
 struct OwnedStrings {
     DevStrings d;
@@ -191,6 +194,7 @@ struct blg_search {
     // and of the queries
     uint64_t *csk = nullptr, *qsk = nullptr;
     uint4 *ccnt = nullptr, *qcnt = nullptr;
+    uint32_t *csig = nullptr, *qsig = nullptr;   // 4-gram signatures (blg_sig.cuh) of the same strings
     void *sk_mem = nullptr;           // the queries' sketch block when this search owns it
     // choices in tile-transposed form (exact and unsorted runs), when the
     // padding to each tile's longest choice stays small
@@ -1216,8 +1220,8 @@ static int search_upload_choices(blg_ctx *c, const uint8_t *bc, const int64_t *o
             auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
             const size_t o_perm = 0, o_tab = up(sizeof(int32_t) * (size_t)nc),
                          o_soff = o_tab + up(sizeof(int64_t) * (size_t)(2 * n_len + 1)),
-                         o_csk = o_soff + up(sizeof(int64_t) * (size_t)(nc + 1)),
-                         o_ccnt = o_csk + up(sizeof(uint64_t) * (size_t)nc),
+                         o_csig = o_soff + up(sizeof(int64_t) * (size_t)(nc + 1)),
+                         o_ccnt = o_csig + up(sizeof(uint32_t) * kSigWords * (size_t)nc),
                          o_buf = o_ccnt + up(sizeof(uint4) * (size_t)nc),
                          total = o_buf + (size_t)bytes + kSlackBefore + kSlackAfter;
             CK(dev_alloc(c, &s->sorted_mem, total), "cudaMallocAsync(sorted choices)");
@@ -1226,7 +1230,7 @@ static int search_upload_choices(blg_ctx *c, const uint8_t *bc, const int64_t *o
             s->lstart = (int64_t *)(m + o_tab);
             int64_t *d_bstart = s->lstart + (n_len + 1);
             int64_t *d_soff = (int64_t *)(m + o_soff);
-            s->csk = (uint64_t *)(m + o_csk);
+            s->csig = (uint32_t *)(m + o_csig);
             s->ccnt = (uint4 *)(m + o_ccnt);
             uint8_t *d_buf = m + o_buf;
             CK(cudaMemcpyAsync(s->perm, perm, sizeof(int32_t) * nc, cudaMemcpyHostToDevice, c->stream), "H2D perm");
@@ -1247,12 +1251,10 @@ static int search_upload_choices(blg_ctx *c, const uint8_t *bc, const int64_t *o
             cs.d.n = nc;
             cs.d.base = 0;
             cs.d.bytes = bytes;
-            CK(launch(c, "gather_strings", [&] {
-                   return launch_gather_strings(c->stream, c->sms, s->c.d, s->perm, cs.d.off,
-                                                (uint8_t *)cs.d.buf, nc, c->d_status);
-               }), "gather_strings");
-            CK(launch(c, "sketch", [&] { return launch_sketch_strings(c->stream, c->sms, cs.d, s->csk, s->ccnt, c->d_status); }),
-               "sketch");
+            CK(launch(c, "gather_sketch", [&] {
+                   return launch_sketch_strings(c->stream, c->sms, s->c.d, s->perm, cs.d.off, (uint8_t *)cs.d.buf, s->csig,
+                                                s->ccnt, c->d_status);
+               }), "gather_sketch");
             s->min_len = mn;
             s->n_len = n_len;
             s->lsorted = true;
@@ -1316,12 +1318,14 @@ static int search_upload_queries(blg_ctx *c, const uint8_t *bq, const int64_t *o
     int rc = upload_strings(c, bq, oq, nq, s->q);
     if (rc) return rc;
     if ((need & NEED_TT) && nq > 0) query_symbols(bq, oq, nq, s);
-    // one block: the sketches (8 B each), then the 4-gram counts (16 B each, 16-byte aligned)
-    const size_t nq1 = (size_t)std::max<int64_t>(nq, 1), o_cnt = (8 * nq1 + 15) & ~size_t(15);
-    CK(dev_alloc(c, (void **)&s->qsk, o_cnt + 16 * nq1), "cudaMallocAsync(sketches)");
-    s->sk_mem = s->qsk;
-    s->qcnt = (uint4 *)((uint8_t *)s->qsk + o_cnt);
-    CK(launch(c, "sketch", [&] { return launch_sketch_strings(c->stream, c->sms, s->q.d, s->qsk, s->qcnt, c->d_status); }),
+    if (!(need & NEED_SORTED)) return BLG_OK;
+    // one block: the signatures (32 B each), then the 4-gram counts (16 B each)
+    const size_t nq1 = (size_t)std::max<int64_t>(nq, 1), o_cnt = sizeof(uint32_t) * kSigWords * nq1;
+    CK(dev_alloc(c, &s->sk_mem, o_cnt + 16 * nq1), "cudaMallocAsync(sketches)");
+    s->qsig = (uint32_t *)s->sk_mem;
+    s->qcnt = (uint4 *)((uint8_t *)s->sk_mem + o_cnt);
+    CK(launch(c, "sketch", [&] { return launch_sketch_strings(c->stream, c->sms, s->q.d, nullptr, nullptr, nullptr, s->qsig, s->qcnt,
+                                                         c->d_status); }),
        "sketch");
     return BLG_OK;
 }
@@ -1466,6 +1470,14 @@ static SurvClasses seq_classes(blg_search *s) {
     return C;
 }
 
+// The longest sequential query of the current classes (in order of words, each by length).
+static int64_t longest_query(const blg_search *s) {
+    int64_t m = 0;
+    for (auto &k_ : s->cls)
+        if (!k_.lanes && !k_.h_qlen.empty()) m = k_.h_qlen.back();
+    return m;
+}
+
 // Queries in the search's current classes (every query of the rows they
 // were built for, empty ones included).
 static int64_t class_queries(const blg_search *s) {
@@ -1505,6 +1517,81 @@ static bool bits_faster(const blg_ctx *c, const blg_search *s) {
         word += 5.0 + std::max(floor, 1.12e-6 * avg * k.nw * (double)k.nq * (double)s->nc);
     }
     return bits <= word;
+}
+
+// Whether a thresholded run of the sequential classes filters on the tensor
+// cores (k_filter_pairs): its tiles, 128 queries x 256 choices over the whole
+// length range of the tile's queries, against the pairs that the per-pair
+// filter would look at. Measured (GB300, k = 2, 4096 x 65536 reads of 64: 474
+// us for 268 M pairs, 0.57 SM clocks a pair; a tile 1024 and more): a tile has
+// to hold 1800 such pairs. And the signatures must be able to tell: with g
+// grams a string fills p = 1 - exp(-g / bins) of its bins and two unrelated
+// strings differ in 2 p (1 - p) of them, give or take the binomial
+// deviation; the share below 8 k passes to the list, which has to stay well
+// within its room. Half the bins where that lets hardly more through: half the
+// product and half the rows to write.
+struct FilterPlan {
+    bool pays = false, folded = false;
+    int nq = 0;
+    double filter_us = 0.0;
+};
+
+// The share of unrelated pairs of m-byte strings that pass at k, per length and
+// per number of bins from tables made once (a plan is part of every call).
+struct PassShare {
+    static constexpr int kLen = 512, kSteps = 64;
+    float mean[2][kLen + 1], rsd[2][kLen + 1], tail[kSteps];
+    PassShare() {
+        const double bins[2] = {(double)kSigBins, (double)kSigBins / 2 - 4};
+        for (int h = 0; h < 2; h++)
+            for (int m = 0; m <= kLen; m++) {
+                const double p = 1.0 - std::exp(-std::max(0, m - 3) / bins[h]), x = 2.0 * p * (1.0 - p);
+                mean[h][m] = (float)(x * bins[h]);
+                rsd[h][m] = (float)(1.0 / std::sqrt(std::max(1.0, bins[h] * x * (1.0 - x))));
+            }
+        for (int i = 0; i < kSteps; i++) tail[i] = (float)(0.5 * std::erfc(i / 8.0 / 1.41421356));   // beyond i / 8 deviations
+    }
+    double operator()(int m, int half, int k) const {
+        m = std::min(m, kLen);
+        const float z = (mean[half][m] - 8.0f * (float)k) * rsd[half][m];
+        if (z <= 0.0f) return 1.0 - tail[std::min(kSteps - 1, (int)(-z * 8.0f))];
+        return tail[std::min(kSteps - 1, (int)(z * 8.0f))];
+    }
+};
+
+static FilterPlan filter_plan(const blg_ctx *c, const blg_search *s, const SurvClasses &C, int k) {
+    static const PassShare pass_share;
+    FilterPlan f;
+    if (k > kSigMaxK || !s->csig || C.n == 0 || (double)s->nq * (double)s->nc < kFltMinPairs) return f;
+    std::vector<int32_t> len;
+    for (auto &q : s->cls)
+        if (!q.lanes) len.insert(len.end(), q.h_qlen.begin(), q.h_qlen.end());
+    const size_t nq = len.size(), tiles_q = (nq + 127) / 128;
+    if (tiles_q > (size_t)kFltMaxTiles) return f;
+    auto window = [&](int64_t m0, int64_t m1) {
+        const int64_t a = std::max<int64_t>(0, std::min(m0 - k - s->min_len, s->n_len));
+        const int64_t b = std::max<int64_t>(a, std::min(m1 + k - s->min_len + 1, s->n_len));
+        return s->h_lstart[b] - s->h_lstart[a];
+    };
+    double pairs = 0.0, tiles = 0.0, pass = 0.0, pass_folded = 0.0;
+    for (size_t t = 0; t < tiles_q; t++) {
+        const size_t q0 = t * 128, q1 = std::min(nq, q0 + 128);
+        for (size_t q = q0; q < q1;) {                       // queries of one length share a window
+            size_t e = q;
+            while (e < q1 && len[e] == len[q]) e++;
+            const double n = (double)(e - q) * (double)window(len[q], len[q]);
+            pairs += n;
+            pass += n * pass_share(len[q], 0, k);
+            pass_folded += n * pass_share(len[q], 1, k);
+            q = e;
+        }
+        tiles += std::ceil((double)window(len[q0], len[q1 - 1]) / 256.0);
+    }
+    f.nq = (int)nq;
+    f.folded = pass_folded <= pass + 1e-4 * pairs;
+    f.filter_us = 6.0 + std::ceil(tiles / c->sms) * (f.folded ? 0.75 : 1.15);
+    f.pays = pairs >= 1800.0 * tiles && pairs >= kFltMinPairs && pass <= (double)c->pl_cap / 16.0;
+    return f;
 }
 
 // The exact run of every sequential query, bit-sliced (k_search_bits).
@@ -1566,13 +1653,45 @@ static int search_run(blg_ctx *c, blg_search *s, int k, int dtype, void *d_out, 
         const SurvClasses C = seq_classes(s);
         const bool band = k <= 31 && C.n > 0;
         const int job = band ? survivor_job_size(c, s, k) : 1024;
+        const FilterPlan fp = band ? filter_plan(c, s, C, k) : FilterPlan{};
+        const bool filter = fp.pays;
+        if (filter) {
+            // the filter, which fills the output beside it; the passers, in place
+            // where the fill ends with the filter, else listed; the listed results;
+            // the whole search in place if a list ran full
+            const PasserList P{c->pl + 4, c->pl, c->pl_cap};
+            const bool whole_fill = (double)whole.n * (double)dtype_size(dtype) / 7.3e6 <= fp.filter_us + 10.0;
+            const ResultList L = whole_fill ? ResultList{nullptr, nullptr, 0} : ResultList{c->rl_hdr + 2, c->rl_hdr, c->rl_cap};
+            const RepairPlan plan{s->lstart, s->min_len, s->n_len, job, ResultList{nullptr, c->pl + 2, 0}};
+            CK(cudaMemsetAsync(c->pl, 0, 4 * sizeof(unsigned long long), c->stream), "clear list");
+            if (!whole_fill) CK(cudaMemsetAsync(c->rl_hdr, 0, sizeof(unsigned long long), c->stream), "clear list");
+            CK(launch(c, "filter_pairs", [&] {
+                   return launch_filter_pairs(c->stream, c->sms, C, fp.nq, s->qsig, s->csig, fp.folded, s->lstart, s->min_len,
+                                              s->n_len, k, P, whole, whole_fill, c->d_status);
+               }), "filter_pairs");
+            CK(launch(c, "solve_passers", [&] {
+                   return launch_solve_passers(c->stream, c->sms, C, s->q.d, s->cs.d, s->perm, s->ccnt, s->qcnt,
+                                               longest_query(s), k, dtype, d_out, s->nc, P, L,
+                                               whole_fill ? BatchFill{nullptr, 0, dtype, 0} : whole, plan, c->d_status);
+               }), "solve_passers");
+            if (!whole_fill)
+                CK(launch(c, "solve_finish", [&] {
+                       return launch_solve_finish(c->stream, c->sms, C, k, P, L, whole, plan);
+                   }), "solve_finish");
+            CK(launch(c, "search_band_repair", [&] {
+                   return launch_search_band(c->stream, c->sms, surv_ctas(c, k), surv_round(c, k), job, C, s->cs.d,
+                                             s->perm, s->ccnt, s->qcnt, k, dtype, d_out, s->nc, nullptr, &plan.gate, nullptr,
+                                             c->d_status);
+               }), "search_band_repair");
+        }
         if (!band)
             CK(launch(c, "fill", [&] { return launch_fill(c->stream, c->sms, whole.out, whole.n, dtype, fillv); }),
                "fill");
-        CK(launch(c, "surv_plan", [&] {
-               return launch_surv_plan(c->stream, C, s->lstart, s->min_len, s->n_len, k, job);
-           }), "surv_plan");
-        if (band) {
+        if (!filter)
+            CK(launch(c, "surv_plan", [&] {
+                   return launch_surv_plan(c->stream, C, s->lstart, s->min_len, s->n_len, k, job);
+               }), "surv_plan");
+        if (band && !filter) {
             const ResultList L{c->rl_hdr + 2, c->rl_hdr, c->rl_cap};
             const FillItems F{nullptr, nullptr, 0, whole, fill_items_of(whole), c->rl_hdr + 1};
             CK(cudaMemsetAsync(c->rl_hdr, 0, 2 * sizeof(unsigned long long), c->stream), "clear list");
@@ -1588,7 +1707,7 @@ static int search_run(blg_ctx *c, blg_search *s, int k, int dtype, void *d_out, 
                                              s->perm, s->ccnt, s->qcnt, k, dtype, d_out, s->nc, nullptr, &L, nullptr,
                                              c->d_status);
                }), "search_band_repair");
-        } else {
+        } else if (!band) {
             for (int i = 0; i < C.n; i++)
                 CK(launch(c, "search_surv", [&] {
                        return launch_search_surv(c->stream, c->sms, C.cls[i].nw, s->cs.d, s->perm, C.cls[i], C.lo[i],
@@ -1728,18 +1847,40 @@ static int search_matches_list(blg_ctx *c, blg_search *s, int k, blg_match *d_ou
     if (C.n == 0 || C.n != (int)s->cls.size()) return BLG_OK;    // a lane-spread class: the dense path
     if (class_queries(s) != s->nq) return BLG_OK;                  // not every query's class: the dense path
     const int job = survivor_job_size(c, s, k);
-    CK(launch(c, "surv_plan", [&] { return launch_surv_plan(c->stream, C, s->lstart, s->min_len, s->n_len, k, job); }),
-       "surv_plan");
     const ResultList L{c->rl_hdr + 2, c->rl_hdr, c->rl_cap};
-    const FillItems F{nullptr, nullptr, 0, BatchFill{nullptr, 0, BLG_UINT8, 0}, 0, c->rl_hdr + 1};
     CK(cudaMemsetAsync(c->rl_hdr, 0, 2 * sizeof(unsigned long long), c->stream), "clear list");
-    CK(launch(c, "search_band_list", [&] {
-           return launch_search_band(c->stream, c->sms, surv_ctas(c, k), surv_round(c, k), job, C, s->cs.d, s->perm,
-                                     s->ccnt, s->qcnt, k, BLG_UINT8, nullptr, s->nc, nullptr, &L, &F, c->d_status);
-       }), "search_band_list");
     unsigned long long cnt = 0;
-    CK(cudaMemcpyAsync(&cnt, c->rl_hdr, sizeof(cnt), cudaMemcpyDeviceToHost, c->stream), "D2H list count");
-    CK(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
+    bool listed = false;
+    const FilterPlan fp = filter_plan(c, s, C, k);
+    if (fp.pays) {
+        const PasserList P{c->pl + 4, c->pl, c->pl_cap};
+        const BatchFill none{nullptr, 0, BLG_UINT8, 0};
+        unsigned long long passers = 0;
+        CK(cudaMemsetAsync(c->pl, 0, 4 * sizeof(unsigned long long), c->stream), "clear list");
+        CK(launch(c, "filter_pairs", [&] {
+               return launch_filter_pairs(c->stream, c->sms, C, fp.nq, s->qsig, s->csig, fp.folded, s->lstart, s->min_len,
+                                          s->n_len, k, P, none, true, c->d_status);
+           }), "filter_pairs");
+        CK(launch(c, "solve_passers", [&] {
+               return launch_solve_passers(c->stream, c->sms, C, s->q.d, s->cs.d, s->perm, s->ccnt, s->qcnt, longest_query(s),
+                                           k, BLG_UINT8, nullptr, s->nc, P, L, none, RepairPlan{}, c->d_status);
+           }), "solve_passers");
+        CK(cudaMemcpyAsync(&passers, c->pl, sizeof(passers), cudaMemcpyDeviceToHost, c->stream), "D2H passers");
+        CK(cudaMemcpyAsync(&cnt, c->rl_hdr, sizeof(cnt), cudaMemcpyDeviceToHost, c->stream), "D2H list count");
+        CK(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
+        listed = passers <= c->pl_cap;                             // else: the per-pair filter
+    }
+    if (!listed) {
+        const FillItems F{nullptr, nullptr, 0, BatchFill{nullptr, 0, BLG_UINT8, 0}, 0, c->rl_hdr + 1};
+        CK(launch(c, "surv_plan", [&] { return launch_surv_plan(c->stream, C, s->lstart, s->min_len, s->n_len, k, job); }),
+           "surv_plan");
+        CK(launch(c, "search_band_list", [&] {
+               return launch_search_band(c->stream, c->sms, surv_ctas(c, k), surv_round(c, k), job, C, s->cs.d, s->perm,
+                                         s->ccnt, s->qcnt, k, BLG_UINT8, nullptr, s->nc, nullptr, &L, &F, c->d_status);
+           }), "search_band_list");
+        CK(cudaMemcpyAsync(&cnt, c->rl_hdr, sizeof(cnt), cudaMemcpyDeviceToHost, c->stream), "D2H list count");
+        CK(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
+    }
     if (cnt > c->rl_cap) return BLG_OK;                            // ran full: the dense path
     std::vector<unsigned long long> e(cnt);
     if (cnt) {
@@ -1797,6 +1938,7 @@ static void search_release(blg_ctx *c, blg_search *s) {
     dev_free(c, s->sk_mem);
     s->sk_mem = nullptr;
     s->csk = s->qsk = nullptr;
+    s->csig = s->qsig = nullptr;
     s->ccnt = s->qcnt = nullptr;
     s->tt_words = nullptr;
     s->tt_base = nullptr;
@@ -2687,6 +2829,10 @@ int blg_init(int device, blg_ctx **out) {
     // result <= max_dist of a launch; more run the in-place repair launch
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->rl_hdr, sizeof(unsigned long long) * (2 + (1u << 20)));
     if (e == cudaSuccess) c->rl_cap = 1u << 20;
+    // the tensor-core filter's passers (32 MB): 2^22 pairs of a launch; more run
+    // the whole search in place
+    if (e == cudaSuccess) e = cudaMalloc((void **)&c->pl, sizeof(unsigned long long) * (4 + (1u << 22)));
+    if (e == cudaSuccess) c->pl_cap = 1u << 22;
     if (e == cudaSuccess) e = cudaEventCreate(&c->t0);
     if (e == cudaSuccess) e = cudaEventCreate(&c->t1);
     if (e == cudaSuccess) {
@@ -2719,6 +2865,7 @@ void blg_destroy(blg_ctx *c) {
     c->model = nullptr;
     if (c->d_status) cudaFree(c->d_status);
     if (c->rl_hdr) cudaFree(c->rl_hdr);
+    if (c->pl) cudaFree(c->pl);
     if (c->t0) cudaEventDestroy(c->t0);
     if (c->t1) cudaEventDestroy(c->t1);
     if (c->stage_done) cudaEventDestroy(c->stage_done);

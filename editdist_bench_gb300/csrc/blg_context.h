@@ -65,6 +65,10 @@ struct blg_ctx {
     // claimed], then rl_cap entries (allocated at init)
     unsigned long long *rl_hdr = nullptr;
     unsigned long long rl_cap = 0;
+    // the tensor-core filter's passers: [count, fill items claimed, the repair
+    // launch's gate, -], then pl_cap entries (allocated at init)
+    unsigned long long *pl = nullptr;
+    unsigned long long pl_cap = 0;
     size_t stage_bytes = 0;
     cudaEvent_t stage_done = nullptr;
     std::vector<ProfRec> prof_recs;

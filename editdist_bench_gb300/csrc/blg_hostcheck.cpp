@@ -16,6 +16,7 @@
 
 #include "blg_bits.cuh"
 #include "blg_device.cuh"
+#include "blg_sig.cuh"
 
 using namespace blg;
 
@@ -321,4 +322,42 @@ extern "C" void blg_host_bits(const uint8_t *buf, const int64_t *off, int nq, co
         const int cnt = (int)((lo[q & 7] >> (q & 24) & 0xffu) | (hi[q & 7] >> (q & 24) & 0xffu) << 8);
         out[q] = n - (int)(off[q + 1] - off[q]) + cnt;
     }
+}
+
+// Signatures of two strings and the product of their e4m3 rows: the sum whose
+// sign k_filter_pairs reads (valid: bit 0 the query's row, bit 1 the choice's;
+// bit 2: half the bins); *diff receives |X ^ Y|.
+extern "C" float blg_host_sig_sum(const uint8_t *x, int m, const uint8_t *y, int n, int k, int valid, int *diff) {
+    auto value = [](uint32_t b) {
+        const int e = (int)(b >> 3 & 15u), f = (int)(b & 7u);
+        float v = e ? 1.0f + (float)f / 8.0f : (float)f / 8.0f;
+        for (int i = e ? e : 1; i > 7; i--) v *= 2.0f;
+        for (int i = e ? e : 1; i < 7; i++) v *= 0.5f;
+        return b & 0x80u ? -v : v;
+    };
+    uint32_t s[2][kSigWords] = {{0}, {0}};
+    const uint8_t *p[2] = {x, y};
+    const int len[2] = {m, n};
+    int bits[2] = {0, 0};
+    const int words = valid & 4 ? 32 : 64;
+    for (int t = 0; t < 2; t++) {
+        for (int i = 0; i + 3 < len[t]; i++) {
+            const uint32_t b = sig_bit((uint32_t)p[t][i] << 24 | (uint32_t)p[t][i + 1] << 16 | (uint32_t)p[t][i + 2] << 8 | p[t][i + 3]);
+            if (valid >> t & 1) s[t][b >> 5] |= 1u << (b & 31);
+        }
+        if (valid & 4) sig_fold(s[t]);
+        for (int w = 0; w < words / 8; w++) bits[t] += popc32(s[t][w]);
+    }
+    *diff = 0;
+    for (int w = 0; w < words / 8; w++) *diff += popc32(s[0][w] ^ s[1][w]);
+    uint32_t ql, qh, cl, ch;
+    sig_query_tail(bits[0], valid & 1, ql, qh);
+    sig_choice_tail(bits[1], k, valid & 2, cl, ch);
+    float sum = 0.0f;
+    for (int w = 0; w < words; w++) {
+        const uint32_t a = w == words - 2 ? ql : w == words - 1 ? qh : sig_query_word(s[0], w >> 3, w & 7);
+        const uint32_t b = w == words - 2 ? cl : w == words - 1 ? ch : sig_choice_word(s[1], w >> 3, w & 7);
+        for (int i = 0; i < 32; i += 8) sum += value(a >> i & 0xffu) * value(b >> i & 0xffu);
+    }
+    return sum;
 }

@@ -551,69 +551,14 @@ __global__ void __launch_bounds__(256) k_fill(void *out, int64_t n, int dtype, u
     fill_share(out, n, dtype, v, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
 }
 
-// dst string i = src string perm[i]; one warp per string, byte-wise copy.
-__global__ void __launch_bounds__(256) k_gather_strings(DevStrings src, const int32_t *perm,
-                                                        const int64_t *dst_off, uint8_t *dst, int64_t n,
-                                                        uint32_t *status) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t i = warp; i < n; i += nwarps) {
-        int len;
-        const uint8_t *p = string_at(src, perm[i], len, status);
-        uint8_t *q = dst + dst_off[i];
-        const int64_t cap = dst_off[i + 1] - dst_off[i];
-        if (len > cap) len = (int)cap;
-        for (int x = lane; x < len; x += 32) q[x] = p[x];
-    }
-}
-
-// Per class (one block each): survivor range [lo, hi) of every query
-// (queries sorted by length), tile counts, and their exclusive prefix
-// tile_start[0..nq]; the class's work counter cleared. The scan walks the
-// queries 1024 at a time.
+// The survivor plan (surv_plan_class), a block per class.
 __global__ void __launch_bounds__(1024) k_surv_plan(SurvClasses C, const int64_t *lstart, int64_t min_len,
                                                     int64_t n_len, int k, int tile) {
     __shared__ __align__(16) unsigned char s_raw[sizeof(SurvClasses)];   // (no constructor runs on shared memory)
     SurvClasses &s_c = *reinterpret_cast<SurvClasses *>(s_raw);
-    __shared__ int64_t s_sum[1024];
-    __shared__ int64_t s_carry;
-    if (threadIdx.x == 0) {
-        s_c = C;
-        s_carry = 0;
-    }
+    if (threadIdx.x == 0) s_c = C;
     __syncthreads();
-    const SearchClass &cls = s_c.cls[blockIdx.x];
-    int32_t *lo = s_c.lo[blockIdx.x], *hi = s_c.hi[blockIdx.x];
-    int64_t *tile_start = s_c.tile_start[blockIdx.x];
-    if (threadIdx.x == 0) *s_c.work[blockIdx.x] = 0;
-    for (int base = 0; base < cls.nq; base += 1024) {
-        const int qi = base + threadIdx.x;
-        int64_t tiles = 0;
-        if (qi < cls.nq) {
-            const int64_t m = cls.qlen[qi];
-            int64_t a = m - k - min_len, b = m + k - min_len + 1;   // length window, index space
-            a = a < 0 ? 0 : (a > n_len ? n_len : a);
-            b = b < 0 ? 0 : (b > n_len ? n_len : b);
-            const int64_t l = lstart[a], h = b > a ? lstart[b] : l;
-            lo[qi] = (int32_t)l;
-            hi[qi] = (int32_t)h;
-            tiles = (h - l + tile - 1) / tile;
-        }
-        s_sum[threadIdx.x] = tiles;
-        __syncthreads();
-        for (int off = 1; off < 1024; off <<= 1) {                     // inclusive scan
-            const int64_t v = threadIdx.x >= off ? s_sum[threadIdx.x - off] : 0;
-            __syncthreads();
-            s_sum[threadIdx.x] += v;
-            __syncthreads();
-        }
-        if (qi < cls.nq) tile_start[qi] = s_carry + s_sum[threadIdx.x] - tiles;
-        __syncthreads();
-        if (threadIdx.x == 0) s_carry += s_sum[1023];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) tile_start[cls.nq] = s_carry;
+    surv_plan_class(s_c, blockIdx.x, lstart, min_len, n_len, k, tile);
 }
 
 // Persistent: every CTA pulls tiles from the device work counter until the
@@ -881,15 +826,6 @@ cudaError_t launch_sorted_offsets(cudaStream_t st, int sms, const int64_t *lstar
     if (n < 0 || n_len <= 0) return cudaSuccess;
     const int64_t blocks = std::min<int64_t>((n + 256) / 256, (int64_t)sms * 8);
     k_sorted_offsets<<<(unsigned)blocks, 256, 0, st>>>(lstart, n_len, min_len, bstart, n, soff);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_gather_strings(cudaStream_t st, int sms, const DevStrings &src, const int32_t *perm,
-                                  const int64_t *dst_off, uint8_t *dst, int64_t n, uint32_t *status) {
-    if (n <= 0) return cudaSuccess;
-    int64_t blocks = (n + 7) / 8;
-    blocks = blocks > (int64_t)sms * 32 ? (int64_t)sms * 32 : blocks;
-    k_gather_strings<<<(unsigned)blocks, 256, 0, st>>>(src, perm, dst_off, dst, n, status);
     return cudaGetLastError();
 }
 

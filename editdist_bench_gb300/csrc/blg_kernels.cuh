@@ -856,6 +856,52 @@ __device__ __forceinline__ int upper_index(const int64_t *pre, int n, int64_t x)
     return a;
 }
 
+// Survivor plan of class c by one block (1024 threads at most): range [lo, hi)
+// of every query (queries sorted by length), tile counts, and their exclusive
+// prefix tile_start[0..nq]; the class's work counter cleared. The scan walks
+// the queries a block's width at a time.
+__device__ __forceinline__ void surv_plan_class(const SurvClasses &C, int c, const int64_t *lstart, int64_t min_len,
+                                                int64_t n_len, int k, int tile) {
+    __shared__ int64_t s_sum[1024];
+    __shared__ int64_t s_carry;
+    const SearchClass &cls = C.cls[c];
+    int32_t *lo = C.lo[c], *hi = C.hi[c];
+    int64_t *tile_start = C.tile_start[c];
+    const int T = blockDim.x;
+    if (threadIdx.x == 0) {
+        s_carry = 0;
+        *C.work[c] = 0;
+    }
+    __syncthreads();
+    for (int base = 0; base < cls.nq; base += T) {
+        const int qi = base + threadIdx.x;
+        int64_t tiles = 0;
+        if (qi < cls.nq) {
+            const int64_t m = cls.qlen[qi];
+            int64_t a = m - k - min_len, b = m + k - min_len + 1;   // length window, index space
+            a = a < 0 ? 0 : (a > n_len ? n_len : a);
+            b = b < 0 ? 0 : (b > n_len ? n_len : b);
+            const int64_t l = lstart[a], h = b > a ? lstart[b] : l;
+            lo[qi] = (int32_t)l;
+            hi[qi] = (int32_t)h;
+            tiles = (h - l + tile - 1) / tile;
+        }
+        s_sum[threadIdx.x] = tiles;
+        __syncthreads();
+        for (int off = 1; off < T; off <<= 1) {                     // inclusive scan
+            const int64_t v = threadIdx.x >= off ? s_sum[threadIdx.x - off] : 0;
+            __syncthreads();
+            s_sum[threadIdx.x] += v;
+            __syncthreads();
+        }
+        if (qi < cls.nq) tile_start[qi] = s_carry + s_sum[threadIdx.x] - tiles;
+        __syncthreads();
+        if (threadIdx.x == 0) s_carry += s_sum[T - 1];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) tile_start[cls.nq] = s_carry;
+}
+
 // ---- deferred results and the output fill as work items
 // A survivor kernel that also fills its output with k+1 (fill items taken
 // between survivor jobs, so the HBM-bound fill overlaps the latency-bound

@@ -24,41 +24,54 @@
 
 #include "blg_kernels.cuh"
 #include "blg_sched.h"
+#include "blg_sig.cuh"
 
 namespace blg {
 
-// sketch[i] = gram_sketch(string i), counts[i] = gram_counts(string i),
-// one warp per string: lane l takes the 4-grams starting at l, l + 32, ...
-// (one unaligned 4-byte read each, consecutive across the warp) and counts
-// them in its own 16 byte counters (4 registers); every 255 steps, before a
-// lane counter can wrap, and at the end the counters are folded into
-// saturating totals, then summed over the warp: with plain adds when the
-// string has fewer than 256 grams, else with saturating byte adds.
-// The sketch bits are an OR over the warp. The values equal the per-thread
-// functions' (the same grams, hash and saturation at 255).
-__global__ void __launch_bounds__(256) k_sketch_strings(DevStrings S, uint64_t *sketch, uint4 *counts,
-                                                        uint32_t *status) {
+// sig[8 i ..] = the 4-gram signature of string i (blg_sig.cuh), counts[i] =
+// gram_counts(string i), one warp per string: lane l takes the 4-grams
+// starting at l, l + 32, ... (one unaligned 4-byte read each, consecutive
+// across the warp) and counts them in its own 16 byte counters (4 registers);
+// every 255 steps, before a lane counter can wrap, and at the end the counters
+// are folded into saturating totals, then summed over the warp: with plain
+// adds when the string has fewer than 256 grams, else with saturating byte
+// adds. The signature's bits are set in shared memory, in four copies to
+// spread the lanes. The counts equal the per-thread function's (the same
+// grams, hash and saturation at 255). perm: string i is S's string perm[i],
+// and its bytes are copied to dst + dst_off[i] as they pass (a gather kernel of
+// its own read them twice: 21 us of a one-call search of 100003 lines).
+__global__ void __launch_bounds__(256) k_sketch_strings(DevStrings S, const int32_t *perm, const int64_t *dst_off,
+                                                        uint8_t *dst, uint32_t *sig, uint4 *counts, uint32_t *status) {
+    __shared__ uint32_t s_sig[8][32];                          // warp: [copy][word]
     const int lane = threadIdx.x & 31;
+    uint32_t *my = s_sig[threadIdx.x >> 5];
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < S.n; i += nwarps) {
         int n;
-        const uint8_t *p = string_at(S, i, n, status);
-        uint32_t sk_lo = 0, sk_hi = 0;
+        const uint8_t *p = string_at(S, perm ? (int64_t)perm[i] : i, n, status);
+        uint8_t *q = nullptr;
+        if (perm) {
+            const int64_t at = dst_off[i];
+            n = (int)min((int64_t)n, dst_off[i + 1] - at);
+            q = dst + at;
+        }
+        my[lane] = 0;
+        __syncwarp();
         uint32_t t[4] = {0, 0, 0, 0};                          // saturating totals, bins 4w .. 4w+3
-        for (int c0 = 0; c0 + 3 < n; c0 += 32 * 255) {
+        for (int c0 = 0; c0 < n; c0 += 32 * 255) {
             uint32_t c[4] = {0, 0, 0, 0};                      // this lane's counts of the chunk
-            const int c1 = min(n - 3, c0 + 32 * 255);          // grams starting before c1
+            const int c1 = min(n, c0 + 32 * 255);
             for (int s = c0 + lane; s < c1; s += 32) {
-                const uint32_t g = __byte_perm(load4(p + s), 0u, 0x0123);   // b[s] << 24 | .. | b[s+3]
+                const uint32_t w4 = load4(p + s);
+                if (q) q[s] = (uint8_t)w4;
+                if (s + 3 >= n) continue;
+                const uint32_t g = __byte_perm(w4, 0u, 0x0123);   // b[s] << 24 | .. | b[s+3]
                 const uint32_t h = g * 0x9E3779B1u;
                 const uint32_t bin = h >> 28, inc = 1u << (8 * (bin & 3));
 #pragma unroll
                 for (int w = 0; w < 4; w++) c[w] += (bin >> 2) == (uint32_t)w ? inc : 0u;
-                if (s + 3 < kSketchWindow) {
-                    const uint32_t bit = h >> 26;
-                    if (bit < 32) sk_lo |= 1u << bit;
-                    else sk_hi |= 1u << (bit - 32);
-                }
+                const uint32_t bit = sig_bit(g);
+                atomicOr(my + (lane & 3) * kSigWords + (bit >> 5), 1u << (bit & 31));
             }
 #pragma unroll
             for (int w = 0; w < 4; w++) t[w] = __vaddus4(t[w], c[w]);
@@ -72,12 +85,13 @@ __global__ void __launch_bounds__(256) k_sketch_strings(DevStrings S, uint64_t *
 #pragma unroll
                 for (int w = 0; w < 4; w++) t[w] = __vaddus4(t[w], __shfl_xor_sync(kFull, t[w], off));
         }
-        sk_lo = __reduce_or_sync(kFull, sk_lo);
-        sk_hi = __reduce_or_sync(kFull, sk_hi);
-        if (lane == 0) {
-            sketch[i] = ((uint64_t)sk_hi << 32) | sk_lo;
-            counts[i] = make_uint4(t[0], t[1], t[2], t[3]);
-        }
+        __syncwarp();
+        uint32_t v = my[lane];
+        v |= __shfl_xor_sync(kFull, v, 8);
+        v |= __shfl_xor_sync(kFull, v, 16);
+        if (lane < kSigWords) sig[i * kSigWords + lane] = v;
+        if (lane == 0) counts[i] = make_uint4(t[0], t[1], t[2], t[3]);
+        __syncwarp();
     }
 }
 
@@ -178,11 +192,13 @@ __global__ void __launch_bounds__(256) k_list_scatter(ResultList L, int32_t *wor
 }
 
 // ------------------------------------------------------------- launchers --
-cudaError_t launch_sketch_strings(cudaStream_t st, int sms, const DevStrings &S, uint64_t *sketch, uint4 *counts,
+// perm null: S's strings in place, nothing copied.
+cudaError_t launch_sketch_strings(cudaStream_t st, int sms, const DevStrings &S, const int32_t *perm,
+                                  const int64_t *dst_off, uint8_t *dst, uint32_t *sig, uint4 *counts,
                                   uint32_t *status) {
     if (S.n <= 0) return cudaSuccess;
     const int grid = (int)std::min<int64_t>((S.n + 7) / 8, (int64_t)sms * 8);     // a warp per string
-    k_sketch_strings<<<grid, 256, 0, st>>>(S, sketch, counts, status);
+    k_sketch_strings<<<grid, 256, 0, st>>>(S, perm, dst_off, dst, sig, counts, status);
     return cudaGetLastError();
 }
 
