@@ -93,6 +93,9 @@ cudaError_t launch_search_band(cudaStream_t st, int sms, int ctas_per_sm, int ro
                                const DevStrings &CS, const int32_t *perm, const uint4 *ccnt, const uint4 *qcnt, int k,
                                int dtype, void *out, int64_t nc, const SurvRows *rows, const ResultList *list,
                                const FillItems *fill, uint32_t *status);
+cudaError_t launch_search_small(cudaStream_t st, const SurvClasses &C, const DevStrings &CS, const int32_t *perm,
+                                const uint4 *ccnt, const uint4 *qcnt, int k, int dtype, void *out, int64_t nc,
+                                uint32_t *status);
 cudaError_t launch_surv_plan(cudaStream_t st, const SurvClasses &C, const int64_t *lstart, int64_t min_len,
                              int64_t n_len, int k, int tile);
 cudaError_t launch_search_surv(cudaStream_t st, int sms, int nw, const DevStrings &CS, const int32_t *perm,
@@ -120,6 +123,11 @@ constexpr double kBitsPfxSaving = 0.45;
 constexpr int kPfxMinQueries = 33, kPfxMaxQueries = 64;
 // Tensor-core filter: pairs below which its launch costs more than it saves.
 constexpr double kFltMinPairs = 1e6;
+// Thresholded searches of at most this many pairs run in one launch
+// (k_search_small). One launch / the survivor kernel, microseconds: 1 x 20000
+// words at k = 2 5 / 77, 64 x 20000 DNA of 30 to 120 at k = 2 22 / 42, 30 x 200000
+// (6 M pairs) 50 / 42, words 46 / 58.
+constexpr double kSmallPairs = 4e6;
 
 struct OwnedStrings {
     DevStrings d;
@@ -1433,8 +1441,10 @@ static int pick_qpb(blg_ctx *c, int nw, int nq_cls, int64_t nc) {
 // Launch the current classes' kernels; the max_dist fill covers rows [q0, q1)
 // (all rows by default: the classes hold every query).
 // Survivors per job of the thresholded search: the tuned size, halved
-// (down to 1024) while the run would have fewer than 4 jobs per warp of the
-// persistent grid, so small searches still spread over the GPU. The
+// (down to 128, a warp's scan step) while the run would have fewer than 4 jobs
+// per warp of the persistent grid, so small searches still spread over the GPU
+// (64 x 200000 lines of 3 to 40 bytes at k = 3: 68 us, 115 with jobs of 1024 at
+// the least; 1000 x 100000: 303 and 309). The
 // survivor count comes from the host copies of the length histogram.
 static int survivor_job_size(blg_ctx *c, const blg_search *s, int k) {
     int64_t total = 0;
@@ -1450,7 +1460,7 @@ static int survivor_job_size(blg_ctx *c, const blg_search *s, int k) {
     }
     const int64_t warps = (int64_t)c->sms * surv_ctas(c, k) * 8;
     int job = c->tune.lpt_job;
-    while (job > 1024 && total < 4 * warps * (int64_t)job) job >>= 1;
+    while (job > 128 && total < 4 * warps * (int64_t)job) job >>= 1;
     return job;
 }
 
@@ -1652,8 +1662,16 @@ static int search_run(blg_ctx *c, blg_search *s, int k, int dtype, void *d_out, 
                               fillv};
         const SurvClasses C = seq_classes(s);
         const bool band = k <= 31 && C.n > 0;
-        const int job = band ? survivor_job_size(c, s, k) : 1024;
-        const FilterPlan fp = band ? filter_plan(c, s, C, k) : FilterPlan{};
+        int64_t seq_q = 0;
+        for (int i = 0; i < C.n; i++) seq_q += C.cls[i].nq;
+        const bool small = band && (double)seq_q * (double)s->nc <= kSmallPairs && seq_q <= 65535;
+        if (small)
+            CK(launch(c, "search_small", [&] {
+                   return launch_search_small(c->stream, C, s->cs.d, s->perm, s->ccnt, s->qcnt, k, dtype, d_out, s->nc,
+                                              c->d_status);
+               }), "search_small");
+        const int job = band && !small ? survivor_job_size(c, s, k) : 1024;
+        const FilterPlan fp = band && !small ? filter_plan(c, s, C, k) : FilterPlan{};
         const bool filter = fp.pays;
         if (filter) {
             // the filter, which fills the output beside it; the passers, in place
@@ -1687,11 +1705,11 @@ static int search_run(blg_ctx *c, blg_search *s, int k, int dtype, void *d_out, 
         if (!band)
             CK(launch(c, "fill", [&] { return launch_fill(c->stream, c->sms, whole.out, whole.n, dtype, fillv); }),
                "fill");
-        if (!filter)
+        if (!filter && !small)
             CK(launch(c, "surv_plan", [&] {
                    return launch_surv_plan(c->stream, C, s->lstart, s->min_len, s->n_len, k, job);
                }), "surv_plan");
-        if (band && !filter) {
+        if (band && !filter && !small) {
             const ResultList L{c->rl_hdr + 2, c->rl_hdr, c->rl_cap};
             const FillItems F{nullptr, nullptr, 0, whole, fill_items_of(whole), c->rl_hdr + 1};
             CK(cudaMemsetAsync(c->rl_hdr, 0, 2 * sizeof(unsigned long long), c->stream), "clear list");
@@ -2276,6 +2294,17 @@ static int batch_upload_body(blg_ctx *c, const blg_problem *pr, int nprob, blg_b
     int64_t *pqs_start = (int64_t *)hb(b_peq_start);
     BatchJob *jobs = (BatchJob *)hb(b_jobs);
     BatchFill *fills = (BatchFill *)hb(b_fills);
+    // survivors per work unit: 1024 (the 256-problem batch 0.99 ms per step; 1.30
+    // with 4096), halved down to a warp's scan step of 128 while there would be
+    // fewer than 4 units per warp of the grid. Survivors estimated by lengths
+    // spread evenly over each problem's range.
+    double survivors = 0.0;
+    for (int i = 0; i < nprob; i++)
+        if (work[i] && eligible[i] && b->kk[i] >= 0 && b->kk[i] <= 31)
+            survivors += (double)pr[i].nq * (double)pr[i].nc *
+                         std::min(1.0, (2.0 * b->kk[i] + 1.0) / (double)(prep[i].mx - prep[i].mn + 1));
+    int tile = 1024;
+    while (tile > 128 && survivors < 4.0 * c->sms * 4 * 8 * tile) tile >>= 1;
     int nl = 0, nu = 0, nsk = 0, npq = 0, nj = 0, nf = 0, max_nwc = 1;
     lss_start[0] = ups_start[0] = sks_start[0] = pqs_start[0] = 0;
     // each group's first set of every kind
@@ -2379,7 +2408,7 @@ static int batch_upload_body(blg_ctx *c, const blg_problem *pr, int nprob, blg_b
             j.k = k;
             j.dtype = p.dtype;
             j.nw = cl.nw;
-            j.tile = 1024;                      // survivors per work unit (config 5: 0.99 ms per step; 1.30 with 4096)
+            j.tile = tile;
             j.csk = s->csk;
             j.qsk = s->qsk;
             j.ccnt = s->ccnt;

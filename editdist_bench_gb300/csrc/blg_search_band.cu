@@ -191,7 +191,56 @@ __global__ void __launch_bounds__(256) k_list_scatter(ResultList L, int32_t *wor
     if (cnt > L.cap && blockIdx.x == 0 && threadIdx.x == 0) *work = 0;
 }
 
+// Small searches (a lookup in a word list): one thread per (query, choice) in
+// the choices' length order, one launch and every output element written
+// once. The survivor kernel's five launches (list cleared, plan, search with
+// fill, scatter, repair) and its jobs of a thousand survivors to a warp
+// cost 72 us on one query and 20011 words, whatever the work; this takes 5.
+// Warps whose choices are all out of the length window only store.
+__global__ void __launch_bounds__(128) k_search_small(SurvClasses C, DevStrings CS, const int32_t *perm,
+                                                      const uint4 *ccnt, const uint4 *qcnt, int k, int dtype, void *out,
+                                                      int64_t nc, uint32_t *status) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nc) return;
+    int at = blockIdx.y;                           // the query's place in its class
+    SearchClass cl = C.cls[0];
+#pragma unroll
+    for (int c = 1; c < kSurvClasses; c++)         // (no dynamic index into the parameter block)
+        if (c < C.n && at >= cl.nq) {
+            at -= cl.nq;
+            cl = C.cls[c];
+        }
+    const int64_t row = __ldg(cl.qidx + at);
+    const int m = __ldg(cl.qlen + at);
+    const uint4 cc = __ldg(ccnt + i), qc = __ldg(qcnt + row);
+    const int64_t to = row * nc + perm[i];
+    int n, d = k + 1;
+    const uint8_t *t = string_at(CS, i, n, status);
+    if ((n > m ? n - m : m - n) <= k) {
+        if (m == 0) {
+            d = n;
+        } else if (gram_dist(qc, cc) <= 8u * (uint32_t)k) {
+            const uint64_t *peq = cl.peq + (size_t)at * 256 * cl.nw;
+            const int nw = cl.nw;
+            d = band_distance(m, t, n, k, [&](uint32_t c, int p0) { return peq_window(peq + c * nw, nw, p0); }, Units{1u, 2u});
+        }
+    }
+    store1(out, dtype, to, d);
+}
+
 // ------------------------------------------------------------- launchers --
+cudaError_t launch_search_small(cudaStream_t st, const SurvClasses &C, const DevStrings &CS, const int32_t *perm,
+                                const uint4 *ccnt, const uint4 *qcnt, int k, int dtype, void *out, int64_t nc,
+                                uint32_t *status) {
+    int64_t nq = 0;
+    for (int c = 0; c < C.n; c++) nq += C.cls[c].nq;
+    if (nq <= 0 || nc <= 0) return cudaSuccess;
+    if (nq > 65535 || k < 0 || k > 31) return cudaErrorInvalidValue;
+    k_search_small<<<dim3((unsigned)((nc + 127) / 128), (unsigned)nq), 128, 0, st>>>(C, CS, perm, ccnt, qcnt, k, dtype, out,
+                                                                                    nc, status);
+    return cudaGetLastError();
+}
+
 // perm null: S's strings in place, nothing copied.
 cudaError_t launch_sketch_strings(cudaStream_t st, int sms, const DevStrings &S, const int32_t *perm,
                                   const int64_t *dst_off, uint8_t *dst, uint32_t *sig, uint4 *counts,

@@ -57,9 +57,9 @@ def _sets(rng, nq, nc, lo, hi, alphabet, rate=0.06):
 # partial query and choice tiles, one word class and several, one length and
 # many, the smallest and largest k, odd row sizes
 @pytest.mark.gpu
-@pytest.mark.parametrize("nq,nc,lo,hi,alphabet,k", [(128, 8192, 64, 64, "dna", 2), (300, 5001, 64, 64, "dna", 0),
+@pytest.mark.parametrize("nq,nc,lo,hi,alphabet,k", [(128, 32768, 64, 64, "dna", 2), (900, 5001, 64, 64, "dna", 0),
                                                     (257, 20003, 50, 80, "dna", 4), (1000, 20001, 100, 140, "dna", 3),
-                                                    (260, 4101, 172, 172, "dna", 13), (129, 9000, 18, 18, "text", 1),
+                                                    (260, 16001, 172, 172, "dna", 13), (129, 32001, 18, 18, "text", 1),
                                                     (600, 30011, 20, 60, "text", 2)])
 def test_filter_search(gpu, nq, nc, lo, hi, alphabet, k):
     rng = np.random.default_rng(nq + nc + k)
@@ -113,3 +113,21 @@ def test_filter_one_call_chunks(gpu):
     q, c = _sets(rng, 701, 100003, 64, 64, W.DNA)
     got = gpu.cdist_packed(q, c, max_dist=2, dtype="uint8")
     np.testing.assert_array_equal(got, oracle.saturate(oracle.cross(q, c, 2, threads=16), "uint8"))
+
+
+# one launch for small searches (k_search_small): a lone query, several word
+# classes, empty strings on both sides, every length window from none to all
+@pytest.mark.gpu
+@pytest.mark.parametrize("nq,nc,lo,hi,k", [(1, 1, 5, 5, 1), (1, 20011, 3, 16, 2), (3, 129, 0, 3, 0), (40, 3000, 0, 40, 3),
+                                           (70, 5000, 1, 300, 31), (9, 1000, 500, 530, 9)])
+def test_small_search(gpu, nq, nc, lo, hi, k):
+    rng = np.random.default_rng(nq + nc)
+    q, c = _sets(rng, nq, max(nc, 20), lo, hi, TEXT, 0.2)
+    c = W.take(c, np.arange(nc))
+    want = oracle.cross(q, c, k, threads=4)
+    s = gpu.SearchBatch(q, c)
+    for dt in ("uint8", "uint16", "int32"):
+        got, labels = _run(gpu, s, s.alloc(dt), k)
+        np.testing.assert_array_equal(got, oracle.saturate(want, dt))
+        assert "search_small" in labels, labels
+    np.testing.assert_array_equal(gpu.cdist_packed(q, c, max_dist=k), want)
