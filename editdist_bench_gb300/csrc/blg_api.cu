@@ -74,6 +74,8 @@ cudaError_t launch_solve(cudaStream_t st, int sms, bool hask, const PairsPlan &p
 cudaError_t launch_solve_band(cudaStream_t st, int sms, int ctas_per_sm, const PairsPlan &plan, int k, int dtype, void *out,
                               int32_t *exit_log, int variant, const uint32_t *alpha);
 cudaError_t launch_byte_presence(cudaStream_t st, int sms, const DevStrings &A, const DevStrings &B, uint32_t *mask);
+cudaError_t launch_pairs_reach(cudaStream_t st, int sms, const DevStrings &A, const DevStrings &B, double avg, int k,
+                               int dtype, void *out, uint32_t *status);
 }  // namespace blg
 int sched_model_ensure(blg_ctx *c, blg_sched_model **out);
 cudaError_t launch_mlp_keys(cudaStream_t st, int sms, const blg_sched_model *m, const blg::PairsPlan &plan,
@@ -142,6 +144,7 @@ struct blg_pairs {
     int64_t n = 0;
     int64_t cap[kLongClasses] = {0, 0, 0, 0, 0};
     int64_t short_pairs = 0;      // pairs whose shorter string is at most 32 bytes
+    bool too_long = false;        // a pair's shorter string exceeds 2048 bytes (before trimming)
     bool trusted = false;         // the host pass found every offset pair in order (kernels skip their checks)
     int64_t len_max_side = 0;     // total bytes of the larger side (a or b)
     void *q_items = nullptr;      // all class regions, one allocation
@@ -512,6 +515,7 @@ static int pairs_classify(blg_ctx *c, const int64_t *oa, const int64_t *ob, int6
     // off[0] >= 0 and off[n] >= off[0] were checked above: with every pair in
     // order, every string lies inside the uploaded buffer
     p->trusted = !bad;
+    p->too_long = hist[kLongClasses] > 0;
     int64_t total = 0, above = hist[kLongClasses];
     for (int j = kLongClasses - 1; j >= 0; j--) {
         above += hist[j];
@@ -654,6 +658,20 @@ static bool pairs_use_tile(const blg_ctx *c, const blg_pairs *p) {
     return c->sched == BLG_SCHED_AUTO && 4 * p->short_pairs >= 3 * p->n;
 }
 
+// Furthest-reaching points (k_pairs_reach) under the automatic schedule while k
+// is small: its steps grow with k^2, the banded loop's columns hardly. One
+// kernel / prep, order and banded loop, microseconds: 2^20 pairs of 8 to 256
+// bytes 102 / 244 at k = 2, 159 / 307 at 4, 302 / 385 at 8, 383 / 407 at 10, 474
+// / 436 at 12; 300000 lines of 40 to 100 25 / 79, 41 / 84, 72 / 86, 89 / 87; few
+// pairs, where three launches wait for one another, 20000 of 8 to 256 49 / 121
+// at 12. Against the short-pair tile kernel (2^20 words of 10 to 30) 35 / 48
+// at 2, 46 / 49 at 3, 62 / 50 at 4. Pairs that a kernel would refuse by
+// their trimmed length (shorter string above 2048) take the other paths.
+static bool pairs_use_reach(const blg_ctx *c, const blg_pairs *p, int k, bool tile) {
+    if (k < 0 || c->sched != BLG_SCHED_AUTO || !p->trusted || p->too_long) return false;
+    return k <= (tile ? 2 : p->n <= (1 << 15) ? 16 : 9);
+}
+
 // One launch of the direct pairs path (tile or staged kernel + the long-pair
 // consumer) over strings A, B (a range of the pair set), results at d_out.
 static int pairs_run_direct(blg_ctx *c, blg_pairs *p, const DevStrings &A, const DevStrings &B, bool use_tile,
@@ -701,6 +719,11 @@ static int pairs_run_range(blg_ctx *c, blg_pairs *p, const DevStrings &A, const 
                            void *d_out, int32_t *exit_log) {
     if (A.n == 0) return BLG_OK;
     const bool use_tile = !exit_log && pairs_use_tile(c, p);
+    if (!exit_log && pairs_use_reach(c, p, k, use_tile)) {
+        CK(launch(c, "pairs_solve", [&] { return launch_pairs_reach(c->stream, c->sms, A, B, (double)p->len_max_side / (double)p->n, k, dtype, d_out, c->d_status); }),
+           "pairs_solve");
+        return BLG_OK;
+    }
     if (!use_tile && (c->sched != BLG_SCHED_PLAIN || exit_log))
         return pairs_run_scheduled(c, p, A, B, k, dtype, d_out, exit_log);
     return pairs_run_direct(c, p, A, B, use_tile, k, dtype, d_out);

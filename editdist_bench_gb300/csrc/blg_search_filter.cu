@@ -38,6 +38,7 @@
 #include <algorithm>
 
 #include "blg_kernels.cuh"
+#include "blg_reach.cuh"
 #include "blg_search_filter.h"
 #include "blg_sig.cuh"
 #include "blg_tma.cuh"
@@ -458,16 +459,12 @@ __global__ void __launch_bounds__(kFltThreads, 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(S.tmem), "r"(512) : "memory");
 }
 
-// The listed pairs, a lane each, by furthest-reaching points (Ukkonen 1985;
-// Landau and Vishkin 1989): F(e, d) is the last pattern position that e edits can
-// reach on diagonal d = j - i, F(e, d) = max(F(e-1, d) + 1, F(e-1, d-1),
-// F(e-1, d+1) + 1) extended over equal characters, eight at a time; the
-// distance is the first e with F(e, n - m) = m. A pair takes about k^2 / 2 steps
-// and n / 8 more, where the banded loop (survivor_warp) walks every column of a
-// near-copy with two scattered loads of the query's Peq rows, 32 lanes in 64
-// cache lines: 52,000 passers of 100 to 256 bytes at k = 4 took 84 us that
-// way. The strings are first copied into shared memory; pairs longer than a
-// slot take the banded loop.
+// The listed pairs, a lane each, by furthest-reaching points (blg_reach.cuh),
+// where the banded loop (survivor_warp) walks every column of a near-copy with
+// two scattered loads of the query's Peq rows, 32 lanes in 64 cache lines:
+// 52,000 passers of 100 to 256 bytes at k = 4 took 84 us that way and take 50.
+// The strings are first copied into shared memory; pairs longer than a slot
+// take the banded loop.
 // The filter leaves off filling the output when its tiles are done, long
 // before 1 GiB is written; here a third warp goes on with it, and as the fill
 // may pass an element after its result, results go to a list (list_emit) that
@@ -475,49 +472,6 @@ __global__ void __launch_bounds__(kFltThreads, 1)
 constexpr int kLvThreads = 64;
 constexpr int kLvMaxK = kSigMaxK;
 constexpr int kLvMaxSlot = 1040;                         // bytes; longer strings take the banded loop
-
-// Eight characters at byte offset p of the block's shared memory (words):
-// three words and two funnel shifts (a slot's slack covers the read).
-__device__ __forceinline__ uint2 slot8(const uint32_t *s, uint32_t p) {
-    const uint32_t *w = s + (p >> 2);
-    const uint32_t w0 = w[0], w1 = w[1], w2 = w[2], sh = (p & 3u) * 8u;
-    return make_uint2(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh));
-}
-
-// min(d, k + 1) of the strings at byte offsets a (m characters) and b (n) of s;
-// |n - m| <= k. f: this thread's column of F(e - 1, .), diagonal 0, stride
-// kLvThreads, from -k - 1 to k + 1. One flat loop: an iteration compares eight
-// characters on the lane's diagonal and, where they end the run, moves to its
-// next one. Lanes of a warp are in different runs, so loops within the loop
-// would last as long as the warp's longest run at every step (7400 warp
-// instructions for 32 pairs of 100 to 256 bytes at k = 4, measured).
-__device__ __forceinline__ int furthest_distance(const uint32_t *s, uint32_t a, int m, uint32_t b, int n, int k,
-                                                 int16_t *f) {
-    const int goal = n - m;
-    for (int d = -k - 1; d <= k + 1; d++) f[d * kLvThreads] = -2;
-    int e = 0, d = 0, hi = 0, i = 0, end = min(m, n), left = -2;
-    while (true) {
-        const uint2 x = slot8(s, a + i), y = slot8(s, b + i + d);
-        const uint32_t u = x.x ^ y.x, v = x.y ^ y.y;
-        const int q = u ? (__ffs(u) - 1) >> 3 : v ? 4 + ((__ffs(v) - 1) >> 3) : 8;
-        i = min(i + q, end);
-        if (q == 8 && i < end) continue;
-        if (d == goal && i >= m) return e;
-        const int old = f[d * kLvThreads];
-        f[d * kLvThreads] = (int16_t)i;
-        left = old;
-        if (d++ == hi) {
-            if (++e > k) return k + 1;
-            // the diagonals that a path of k edits to the goal can still be on
-            d = max(max(-e, goal - (k - e)), -m);
-            hi = min(min(e, goal + (k - e)), n);
-            left = f[(d - 1) * kLvThreads];
-        }
-        end = min(m, n - d);                             // the diagonal's last position
-        i = max(max((int)f[d * kLvThreads] + 1, left), (int)f[(d + 1) * kLvThreads] + 1);
-        i = min(i, end);
-    }
-}
 
 // The repair launch's plan and its gate, by the blocks of a launch.
 __device__ __forceinline__ void repair_plan(const SurvClasses &C, const RepairPlan &R, int k) {
@@ -586,7 +540,8 @@ __global__ void __launch_bounds__(kLvThreads + 32)
         int d;
         if (fits) {
             const uint32_t base = (uint32_t)(warp * 64 + 2 * lane) * (uint32_t)slot;
-            d = furthest_distance(reinterpret_cast<const uint32_t *>(s_dyn), base + sa, m, base + slot + sb, n, k, f);
+            const uint32_t *w = reinterpret_cast<const uint32_t *>(s_dyn);
+            d = furthest_distance<kLvThreads>(w, base + sa, m, w, base + slot + sb, n, k, f);
         } else if (m == 0) {
             d = n;
         } else {
