@@ -24,7 +24,7 @@ PROBE = os.path.join(HERE, "libblg_probe.so")
 
 CU_SOURCES = ["blg_api.cu", "blg_kernels.cu", "blg_noalloc.cu", "blg_pairs_sched.cu", "blg_mlp.cu", "blg_batch.cu",
               "blg_pairs_tile.cu", "blg_search_band.cu", "blg_search_bits.cu",
-              "blg_search_filter.cu", "blg_pairs_reach.cu", "blg_matches.cu"]
+              "blg_search_filter.cu", "blg_pairs_reach.cu", "blg_pairs_exact.cu", "blg_matches.cu"]
 HEADERS = ["blg_device.cuh", "blg_internal.h", "blg_kernels.cuh", "blg_context.h", "blg_sched.h", "blg_batch.h", "blg_tma.cuh",
            "blg_bits.cuh", "blg_search_bits.h", "blg_search_filter.h", "blg_sig.cuh",
            "blg_reach.cuh"]

@@ -74,6 +74,9 @@ cudaError_t launch_solve(cudaStream_t st, int sms, bool hask, const PairsPlan &p
 cudaError_t launch_solve_band(cudaStream_t st, int sms, int ctas_per_sm, const PairsPlan &plan, int k, int dtype, void *out,
                               int32_t *exit_log, int variant, const uint32_t *alpha);
 cudaError_t launch_byte_presence(cudaStream_t st, int sms, const DevStrings &A, const DevStrings &B, uint32_t *mask);
+cudaError_t launch_pairs_bands(cudaStream_t st, int sms, const DevStrings &A, const DevStrings &B, int dtype,
+                               void *out, const PairsPlan &plan, LongItem *far, int32_t *nfar, int32_t *left,
+                               int variant, const uint32_t *alpha, uint32_t *status);
 cudaError_t launch_pairs_reach(cudaStream_t st, int sms, const DevStrings &A, const DevStrings &B, double avg, int k,
                                int dtype, void *out, uint32_t *status);
 }  // namespace blg
@@ -158,6 +161,8 @@ struct blg_pairs {
     // known; the banded solver's one-row-per-byte variant needs at most 15)
     uint32_t *d_alpha = nullptr;
     int nsym = -1;
+    // resident sets: a sample's pairs share 4-grams (pairs_related)
+    bool related = false;
     // resident runs as a CUDA graph (pairs_run_graph): the launches of one
     // run, captured once its parameters repeat, replayed while they stay
     struct GraphKey {
@@ -540,7 +545,7 @@ static int pairs_upload(blg_ctx *c, const uint8_t *ba, const int64_t *oa, const 
     return rc;
 }
 
-constexpr size_t kPlanCounters = 2 * kPairClasses;   // count, head
+constexpr size_t kPlanCounters = 2 * kPairClasses + 1;   // count, head; far pairs of an exact run (pairs_run_bands)
 
 static int plan_alloc(blg_ctx *c, blg_pairs *p, bool feat) {
     int64_t slots = 0;
@@ -658,6 +663,68 @@ static bool pairs_use_tile(const blg_ctx *c, const blg_pairs *p) {
     return c->sched == BLG_SCHED_AUTO && 4 * p->short_pairs >= 3 * p->n;
 }
 
+// Whether the pairs of a set are mostly near each other, from 32 of them: their
+// sets of 6-grams (4096 hashed bins) differ in well under what unrelated
+// strings' would; edits at a rate r keep (1 - r)^6 of the grams. Decides a
+// route, never a result.
+static bool pairs_related(const uint8_t *ba, const int64_t *oa, const uint8_t *bb, const int64_t *ob, int64_t n) {
+    constexpr int kGram = 6, kBins = 4096;
+    const int64_t samples = std::min<int64_t>(32, n);
+    double differ = 0.0, expected = 0.0;
+    for (int64_t x = 0; x < samples; x++) {
+        const int64_t i = n * x / samples;
+        uint64_t set[2][kBins / 64] = {};
+        int bits[2] = {0, 0}, diff = 0;
+        for (int t = 0; t < 2; t++) {
+            const uint8_t *p = (t ? bb : ba) + (t ? ob : oa)[i];
+            const int64_t len = std::min<int64_t>(512, (t ? ob : oa)[i + 1] - (t ? ob : oa)[i]);
+            for (int64_t y = 0; y + kGram <= len; y++) {
+                uint32_t h = 0;
+                for (int z = 0; z < kGram; z++) h = (h ^ p[y + z]) * 0x9E3779B1u;
+                set[t][h >> 26] |= 1ull << (h >> 20 & 63u);
+            }
+            for (uint64_t w : set[t]) bits[t] += __builtin_popcountll(w);
+        }
+        for (int w = 0; w < kBins / 64; w++) diff += __builtin_popcountll(set[0][w] ^ set[1][w]);
+        differ += diff;
+        expected += bits[0] + bits[1] - 2.0 * bits[0] * bits[1] / kBins;
+    }
+    return expected > 0.0 && differ < 0.8 * expected;
+}
+
+// Bands first, for exact runs of a resident set (its alphabet and a sample are
+// known) of near pairs with patterns past one word. Bands / full width,
+// microseconds: 250007 pairs of 8 to 256 bytes with up to 30% edits 243 / 355,
+// 10^6 829 / 1197, 250000 of 60 to 120 with up to 10% 81 / 128. Few pairs wait for the
+// longer chain of kernels (20000 of 8 to 256 147 / 120, 100000 172 / 180) unless no
+// pattern is longer than 128 (20000 of 4 to 80 44 / 62); unrelated pairs leave both
+// bands late (60 to 250 bytes: 643 / 470).
+static bool pairs_use_bands(const blg_ctx *c, const blg_pairs *p) {
+    return c->sched == BLG_SCHED_AUTO && p->trusted && !p->too_long && p->cap[0] > 0 && p->nsym >= 0 && p->related &&
+           (p->n >= (1 << 16) || p->cap[1] == 0);
+}
+
+// Exact runs with long patterns under the automatic schedule: bands first
+// (blg_pairs_exact.cu), the pairs beyond them by the full-width solvers.
+static int pairs_run_bands(blg_ctx *c, blg_pairs *p, const DevStrings &A, const DevStrings &B, int dtype, void *d_out) {
+    int rc = plan_alloc(c, p, false);
+    if (rc) return rc;
+    const PairsPlan plan = plan_view(p);
+    CK(cudaMemsetAsync(p->plan_ctr, 0, sizeof(int32_t) * kPlanCounters, c->stream), "reset plan");
+    int variant = -1;
+    rc = pairs_alphabet(c, p, A, B, &variant);
+    if (rc) return rc;
+    CK(launch(c, "pairs_bands", [&] {
+           return launch_pairs_bands(c->stream, c->sms, A, B, dtype, d_out, plan,
+                                     plan.raw[0], p->plan_ctr + 2 * kPairClasses, plan.count, variant, p->d_alpha,
+                                     c->d_status);
+       }), "pairs_bands");
+    CK(launch(c, "pairs_solve", [&] {
+           return launch_solve(c->stream, c->sms, false, plan, -1, dtype, d_out, nullptr, true);
+       }), "pairs_solve");
+    return BLG_OK;
+}
+
 // Furthest-reaching points (k_pairs_reach) under the automatic schedule while k
 // is small: its steps grow with k^2, the banded loop's columns hardly. One
 // kernel / prep, order and banded loop, microseconds: 2^20 pairs of 8 to 256
@@ -724,6 +791,7 @@ static int pairs_run_range(blg_ctx *c, blg_pairs *p, const DevStrings &A, const 
            "pairs_solve");
         return BLG_OK;
     }
+    if (k < 0 && !exit_log && !use_tile && pairs_use_bands(c, p)) return pairs_run_bands(c, p, A, B, dtype, d_out);
     if (!use_tile && (c->sched != BLG_SCHED_PLAIN || exit_log))
         return pairs_run_scheduled(c, p, A, B, k, dtype, d_out, exit_log);
     return pairs_run_direct(c, p, A, B, use_tile, k, dtype, d_out);
@@ -2949,6 +3017,7 @@ int blg_pairs_upload(blg_ctx *c, const uint8_t *ba, const int64_t *oa, const uin
     // synchronises): the device copy is the data the host pass checked,
     // whatever the caller does with its buffers.
     if (!rc) rc = pairs_learn_alphabet(c, p);
+    if (!rc && n > 0 && p->trusted) p->related = pairs_related(ba, oa, bb, ob, n);
     if (!rc && cudaStreamSynchronize(c->stream) != cudaSuccess) rc = fail(c, BLG_ERR_CUDA, "upload");
     if (rc) {
         pairs_release(c, p);

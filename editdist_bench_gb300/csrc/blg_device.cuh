@@ -298,6 +298,46 @@ BLG_HD int band_core(int m, int n, int k, TextFn text, EqW eqw, Units u, int *co
     return exited ? k + 1 : band_finish(k, bg, s);
 }
 
+// The banded run with a 64-row window (k <= 63): the same band, boundaries and
+// exit in 64-bit words. eq4(j, p0, e) sets e[0..3] to the match bits of
+// columns j .. j + 3 (j a multiple of 4; past the text anything), whose windows
+// start at pattern indexes p0 .. p0 + 3: four columns' loads before their
+// chain of dependent steps. Returns min(d, k + 1). Caller guarantees 1 <= m, |n -
+// m| <= k <= 63.
+template <typename Eq4>
+BLG_HD int band64_core(int m, int n, int k, Eq4 eq4) {
+    const int g = n - m, half = (k - (g < 0 ? -g : g)) >> 1;
+    const int dhi = (g > 0 ? g : 0) + half, dlo = (g < 0 ? g : 0) - half, B = dhi - dlo + 1, s = dhi - g;
+    const uint64_t band = (B >= 64 ? ~0ull : ((1ull << B) - 1)) & ~1ull;
+    const int nv = dhi + 1;
+    uint64_t mv = nv >= 64 ? ~0ull : ((1ull << nv) - 1), pv = ~mv;
+    int A = dhi;
+    auto popc64 = [](uint64_t x) { return popc32((uint32_t)x) + popc32((uint32_t)(x >> 32)); };
+    for (int j = 0; j < n; j += 4) {
+        if (j > 0 && A - popc64(mv & band) > k) return k + 1;            // every band cell > k
+        uint64_t e[4];
+        eq4(j, j - dhi, e);
+        const int cols = n - j < 4 ? n - j : 4;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+        for (int x = 0; x < 4; x++) {
+            if (x >= cols) break;
+            pv = (pv >> 1) | (1ull << 63);
+            mv >>= 1;
+            const uint64_t eq = e[x], xv = eq | mv;
+            const uint64_t xh = (((eq & pv) + pv) ^ pv) | eq;
+            const uint64_t ph = mv | ~(xh | pv), mh = pv & xh;
+            const uint64_t phs = (ph << 1) | 1, mhs = mh << 1;
+            pv = mhs | ~(xv | phs);
+            mv = phs & xv;
+            A += 1 + (int)(pv & 1) - (int)(mv & 1);
+        }
+    }
+    const uint64_t ms = (s >= 63 ? ~0ull : ((2ull << s) - 1)) & ~1ull;   // bits 1..s
+    return cap_k(A + popc64(pv & ms) - popc64(mv & ms), k);
+}
+
 // ---- host-side reference of the per-pair device logic ------------------
 // pair_distance_plain: trimming + pattern = shorter string + gap exit +
 // single/multi-word run with per-character Eq from a 256-row table.  The

@@ -361,3 +361,16 @@ extern "C" float blg_host_sig_sum(const uint8_t *x, int m, const uint8_t *y, int
     }
     return sum;
 }
+
+// band64_core with its match bits from the pattern itself.
+extern "C" int blg_host_band64(const uint8_t *a, int m, const uint8_t *b, int n, int k) {
+    return band64_core(m, n, k, [&](int j, int p0, uint64_t (&e)[4]) {
+        for (int x = 0; x < 4; x++) {
+            e[x] = 0;
+            for (int i = 0; i < 64; i++) {
+                const int p = p0 + x + i;
+                if (j + x < n && p >= 0 && p < m && a[p] == b[j + x]) e[x] |= 1ull << i;
+            }
+        }
+    });
+}

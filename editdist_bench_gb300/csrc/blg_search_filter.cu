@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(kLvThreads + 32)
     k_solve_passers(SurvClasses C, DevStrings Q, DevStrings CS, const int32_t *perm, const uint4 *ccnt,
                     const uint4 *qcnt, int k, int dtype, void *out, int64_t nc, int slot, PasserList P, ResultList L,
                     BatchFill fill, RepairPlan plan, uint32_t *status) {
-    extern __shared__ __align__(16) uint8_t s_dyn[];     // per warp [32][2][slot], then F
+    extern __shared__ __align__(16) uint8_t s_dyn[];     // per warp [2][32][slot], then F
     __shared__ __align__(16) uint8_t s_pattern[kFillPiece];
     __shared__ __align__(16) unsigned char s_raw[sizeof(SurvClasses)];
     SurvClasses &SC = *reinterpret_cast<SurvClasses *>(s_raw);
@@ -528,20 +528,20 @@ __global__ void __launch_bounds__(kLvThreads + 32)
         // instructions a warp for what shuffled addresses and whole lines took 1100)
         __syncwarp();
         if (fits) {
-            const uint32_t dst = smem_addr(slots + 2 * lane * slot);
+            const uint32_t dst = smem_addr(slots + lane * slot);
             const uint8_t *pa = a - sa, *pb = b - sb;
             for (int x = 0; x < sa + m; x += 16)
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + x), "l"(pa + x) : "memory");
             for (int x = 0; x < sb + n; x += 16)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + slot + x), "l"(pb + x) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 32 * slot + x), "l"(pb + x) : "memory");
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
         if (!live) continue;
         int d;
         if (fits) {
-            const uint32_t base = (uint32_t)(warp * 64 + 2 * lane) * (uint32_t)slot;
+            const uint32_t base = (uint32_t)(warp * 64 + lane) * (uint32_t)slot;
             const uint32_t *w = reinterpret_cast<const uint32_t *>(s_dyn);
-            d = furthest_distance<kLvThreads>(w, base + sa, m, w, base + slot + sb, n, k, f);
+            d = furthest_distance<kLvThreads>(w, base + sa, m, w, base + 32 * slot + sb, n, k, f);
         } else if (m == 0) {
             d = n;
         } else {
