@@ -9,9 +9,9 @@
 // tcgen05.mma of 128 x 256 x 32 (128 clocks each) and takes about 1750 clocks,
 // 0.05 a pair; the warps that read and write its operands bind (1470 and
 // 1300 clocks of work a tile), not the products. Measured: k = 2 on 4096 x 65536
-// reads of 64, uint8: 76 us a search against 498 of the per-pair filter; k =
+// reads of 64, uint8: 72 us a search against 498 of the per-pair filter; k =
 // 4 on 1024 x 2^20 reads of 100 to 256 (1 GiB of output, 140 us of writing):
-// 209 against 345.
+// 207 against 345.
 //
 // One CTA per SM walks its share of the tiles; its warps have roles and meet
 // on mbarriers:
@@ -48,7 +48,7 @@ namespace blg {
 constexpr int kFltThreads = 640;
 constexpr int kFltReaders = 8;                           // reading warps: 4 .. 11; producing: 12 .. 19
 constexpr int kFltM = 128, kFltN = 256;                  // tile: queries x choices
-constexpr int kFltStage = 512;                           // passers a reading warp buffers
+constexpr int kFltHits = 16;                             // chunks with a passer that a reading warp keeps back
 constexpr int kFillPiece = 4096;                         // bytes of one bulk copy of the fill constant
 constexpr int64_t kFillItem = 65536;                     // bytes claimed at a time
 
@@ -58,7 +58,8 @@ struct __align__(128) FilterShared {
     uint8_t a[kFltM * K];
     uint8_t b[2][kFltN * K];
     uint8_t pattern[kFillPiece];
-    unsigned long long pass[kFltReaders][kFltStage];
+    uint32_t hit[kFltReaders][kFltHits][32];             // per row: the chunk's columns that pass
+    uint2 hit_at[kFltReaders][kFltHits];                 // first row's query, first column's choice
     int64_t start[kFltMaxTiles + 1];                     // first tile of each query tile
     int32_t lo[kFltMaxTiles], hi[kFltMaxTiles];          // its choice range
     uint64_t full[2], empty[2], tfull[2], tempty[2];
@@ -223,7 +224,17 @@ __global__ void __launch_bounds__(kFltThreads, 1)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    fill_pattern(S.pattern, fill);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // the fill starts at once; the others plan first and meet without it
+    if (warp == 1)
+        fill_items(fill, L.count + 1, S.pattern, blockIdx.x == 0,
+                   [&] { return !whole_fill && *(volatile int *)&S.done >= kFltReaders; });
+    auto sync_rest = [] { asm volatile("bar.sync 1, %0;" ::"n"(kFltThreads - 32) : "memory"); };
+    int issued = 0;
+    if (warp != 1) {
     // every query tile's choice range: lengths within k of its shortest and longest query
     for (int t = tid; t < qtiles; t += kFltThreads) {
         int at;
@@ -237,10 +248,7 @@ __global__ void __launch_bounds__(kFltThreads, 1)
         S.lo[t] = (int32_t)lstart[x];
         S.hi[t] = (int32_t)lstart[y];
     }
-    fill_pattern(S.pattern, fill);
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    sync_rest();
     if (warp == 2) {                                     // prefix of the tile counts
         int64_t run = 0;
         for (int t0 = 0; t0 < qtiles; t0 += 32) {
@@ -257,7 +265,7 @@ __global__ void __launch_bounds__(kFltThreads, 1)
         }
         if (lane == 0) S.start[qtiles] = run;
     }
-    __syncthreads();
+    sync_rest();
     const int64_t total = S.start[qtiles];
     const int64_t i0 = total * blockIdx.x / gridDim.x, i1 = total * (blockIdx.x + 1) / gridDim.x;
     const int ntiles = (int)(i1 - i0);
@@ -266,7 +274,6 @@ __global__ void __launch_bounds__(kFltThreads, 1)
         while (i0 + i >= S.start[qt + 1]) qt++;
     };
 
-    int issued = 0;
     if (warp == 0) {
         if (lane == 0) {
             // D f32 | A, B e4m3, both K-major | N | M
@@ -288,77 +295,51 @@ __global__ void __launch_bounds__(kFltThreads, 1)
             }
         }
         __syncwarp();
-    } else if (warp == 1) {
-        fill_items(fill, L.count + 1, S.pattern, blockIdx.x == 0,
-                   [&] { return !whole_fill && *(volatile int *)&S.done >= kFltReaders; });
     } else if (warp >= 4 && warp < 4 + kFltReaders) {
         const int w = warp - 4, rows = (w & 3) * 32, half = (w >> 2) * (kFltN / 2);   // (TMEM rows go by warp mod 4)
-        unsigned long long *stage = S.pass[w];
-        int held = 0;                                    // passers buffered (uniform)
-        auto flush = [&]() {                             // every lane; the warp's buffer to the list
+        int held = 0;                                    // hit chunks kept back (uniform)
+        auto flush = [&]() {                             // every lane; the kept chunks' passers to the list
             __syncwarp();
-            unsigned long long at = 0;
-            if (lane == 0) at = atomicAdd(L.count, (unsigned long long)held);
-            at = __shfl_sync(kFull, at, 0);
-            for (int x = lane; x < held; x += 32)
-                if (at + x < L.cap) L.item[at + x] = stage[x];
-            held = 0;
-            __syncwarp();
-        };
-        // the signs of 32 columns; the pairs with a sum >= 0 (q: the lane's query << 32, c: the first column's choice)
-        auto take = [&](const uint32_t (&v)[32], unsigned long long q, uint32_t c) {
-            uint32_t a[11];
-#pragma unroll
-            for (int x = 0; x < 10; x++) a[x] = v[3 * x] & v[3 * x + 1] & v[3 * x + 2];
-            a[10] = v[30] & v[31];
-            const uint32_t neg = (a[0] & a[1] & a[2]) & (a[3] & a[4] & a[5]) & (a[6] & a[7] & a[8]) & (a[9] & a[10]);
-            const unsigned lanes = __ballot_sync(kFull, (int32_t)neg >= 0);
-            if (!lanes) return;
-            uint32_t mask = 0;                           // sign bits, column x at bit x: four chains of eight shifts
-            if ((int32_t)neg >= 0) {
-                uint32_t b[4] = {0, 0, 0, 0};
-#pragma unroll
-                for (int x = 7; x >= 0; x--)
-#pragma unroll
-                    for (int y = 0; y < 4; y++) b[y] = __funnelshift_l(v[8 * y + x], b[y], 1);
-                mask = ~(b[0] | (b[1] << 8) | (b[2] << 16) | (b[3] << 24));
-            }
-            if (__popc(lanes) <= 4 && held + 4 * 32 <= kFltStage) {
-                // the usual case, a row or two: the reading warps' slowest one holds up the
-                // tile, so no scan over the warp (a passer in two tiles of three: 62 us a
-                // search with the scan)
-                for (unsigned l = lanes; l; l &= l - 1) {
-                    const int src = __ffs(l) - 1;
-                    const uint32_t mk = __shfl_sync(kFull, mask, src);
-                    if (lane == src)
-                        for (int at = held; mask; mask &= mask - 1, at++) stage[at] = q | (c + (uint32_t)(__ffs(mask) - 1));
-                    held += __popc(mk);
-                }
-                __syncwarp();
-                return;
-            }
-            const int n = __popc(mask);
+            int n = 0;
+            for (int x = 0; x < held; x++) n += __popc(S.hit[w][x][lane]);
             int incl = n;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int y = __shfl_up_sync(kFull, incl, o);
                 if (lane >= o) incl += y;
             }
-            const int all = __shfl_sync(kFull, incl, 31);
-            if (held + all > kFltStage && held > 0) flush();
-            unsigned long long g = 0;
-            const bool direct = all > kFltStage;         // more than the buffer holds: straight to the list
-            if (direct) {
-                if (lane == 0) g = atomicAdd(L.count, (unsigned long long)all);
-                g = __shfl_sync(kFull, g, 0);
+            unsigned long long at = 0;
+            if (lane == 31) at = atomicAdd(L.count, (unsigned long long)incl);
+            at = __shfl_sync(kFull, at, 31) + (unsigned long long)(incl - n);
+            for (int x = 0; x < held; x++) {
+                const uint2 h = S.hit_at[w][x];
+                for (uint32_t m = S.hit[w][x][lane]; m; m &= m - 1, at++)
+                    if (at < L.cap) L.item[at] = (unsigned long long)(h.x + lane) << 32 | (h.y + (uint32_t)(__ffs(m) - 1));
             }
-            for (int at = held + incl - n; mask; mask &= mask - 1, at++) {
-                const unsigned long long e = q | (c + (uint32_t)(__ffs(mask) - 1));
-                if (!direct) stage[at] = e;
-                else if (g + at < L.cap) L.item[g + at] = e;
-            }
-            if (!direct) held += all;
+            held = 0;
             __syncwarp();
+        };
+        // the signs of 32 columns of the rows from query q on, columns from choice c
+        // on. A chunk with a pair that passes (a sum >= 0) leaves its columns as a
+        // mask per row, 32 shifts for the warp; the masks become list entries
+        // sixteen chunks at a time, one scan and one atomic for all. The slowest
+        // reading warp holds up the tile: entries made on the spot took 0.9 us a tile
+        // with nine passers, 0.45 with none, a walk of the passing lanes alone 2.2.
+        auto take = [&](const uint32_t (&v)[32], uint32_t q, uint32_t c) {
+            uint32_t a[11];
+#pragma unroll
+            for (int x = 0; x < 10; x++) a[x] = v[3 * x] & v[3 * x + 1] & v[3 * x + 2];
+            a[10] = v[30] & v[31];
+            const uint32_t neg = (a[0] & a[1] & a[2]) & (a[3] & a[4] & a[5]) & (a[6] & a[7] & a[8]) & (a[9] & a[10]);
+            if (!__any_sync(kFull, (int32_t)neg >= 0)) return;
+            uint32_t b[4] = {0, 0, 0, 0};                // sign bits, column x at bit x: four chains of eight shifts
+#pragma unroll
+            for (int x = 7; x >= 0; x--)
+#pragma unroll
+                for (int y = 0; y < 4; y++) b[y] = __funnelshift_l(v[8 * y + x], b[y], 1);
+            S.hit[w][held][lane] = ~(b[0] | (b[1] << 8) | (b[2] << 16) | (b[3] << 24));
+            if (lane == 0) S.hit_at[w][held] = make_uint2(q, c);
+            if (++held == kFltHits) flush();
         };
         for (int i = 0; i < ntiles; i++) {
             const int buf = i & 1;
@@ -366,7 +347,7 @@ __global__ void __launch_bounds__(kFltThreads, 1)
             advance(i);
             __syncwarp();
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const unsigned long long q = (unsigned long long)(qt * kFltM + rows + lane) << 32;
+            const uint32_t q = (uint32_t)(qt * kFltM + rows);
             const uint32_t base = (uint32_t)(S.lo[qt] + (i0 + i - S.start[qt]) * kFltN) + half;
             const uint32_t t0 = S.tmem + ((uint32_t)rows << 16) + buf * kFltN + half;
             uint32_t v0[32], v1[32];
@@ -384,7 +365,6 @@ __global__ void __launch_bounds__(kFltThreads, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive(&S.tempty[buf]);
         }
-        __syncwarp();
         if (held > 0) flush();
         if (lane == 0) atomicAdd(&S.done, 1);
     } else if (warp >= 4 + kFltReaders) {
@@ -449,6 +429,7 @@ __global__ void __launch_bounds__(kFltThreads, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive(&S.full[buf]);
         }
+    }
     }
     // products in flight end before TMEM goes back: the last commits of both buffers
     for (int i = max(0, issued - 2); i < issued; i++) mbar_wait(&S.tfull[i & 1], (uint32_t)(i >> 1) & 1u);
