@@ -208,7 +208,6 @@ struct blg_search {
     std::vector<int64_t> h_lstart;   // host copy of lstart
     // 4-gram sketches and binned 4-gram counts: of the length-sorted choices
     // and of the queries
-    uint64_t *csk = nullptr, *qsk = nullptr;
     uint4 *ccnt = nullptr, *qcnt = nullptr;
     uint32_t *csig = nullptr, *qsig = nullptr;   // 4-gram signatures (blg_sig.cuh) of the same strings
     void *sk_mem = nullptr;           // the queries' sketch block when this search owns it
@@ -700,8 +699,8 @@ static bool pairs_related(const uint8_t *ba, const int64_t *oa, const uint8_t *b
 // pattern is longer than 128 (20000 of 4 to 80 44 / 62); unrelated pairs leave both
 // bands late (60 to 250 bytes: 643 / 470).
 static bool pairs_use_bands(const blg_ctx *c, const blg_pairs *p) {
-    return c->sched == BLG_SCHED_AUTO && p->trusted && !p->too_long && p->cap[0] > 0 && p->nsym >= 0 && p->related &&
-           (p->n >= (1 << 16) || p->cap[1] == 0);
+    return c->sched == BLG_SCHED_AUTO && !c->tuning && p->trusted && !p->too_long && p->cap[0] > 0 && p->nsym >= 0 &&
+           p->related && (p->n >= (1 << 16) || p->cap[1] == 0);
 }
 
 // Exact runs with long patterns under the automatic schedule: bands first
@@ -735,7 +734,7 @@ static int pairs_run_bands(blg_ctx *c, blg_pairs *p, const DevStrings &A, const 
 // at 2, 46 / 49 at 3, 62 / 50 at 4. Pairs that a kernel would refuse by
 // their trimmed length (shorter string above 2048) take the other paths.
 static bool pairs_use_reach(const blg_ctx *c, const blg_pairs *p, int k, bool tile) {
-    if (k < 0 || c->sched != BLG_SCHED_AUTO || !p->trusted || p->too_long) return false;
+    if (k < 0 || c->sched != BLG_SCHED_AUTO || c->tuning || !p->trusted || p->too_long) return false;
     return k <= (tile ? 2 : p->n <= (1 << 15) ? 16 : 9);
 }
 
@@ -1663,7 +1662,7 @@ struct PassShare {
 static FilterPlan filter_plan(const blg_ctx *c, const blg_search *s, const SurvClasses &C, int k) {
     static const PassShare pass_share;
     FilterPlan f;
-    if (k > kSigMaxK || !s->csig || C.n == 0 || (double)s->nq * (double)s->nc < kFltMinPairs) return f;
+    if (c->tuning || k > kSigMaxK || !s->csig || C.n == 0 || (double)s->nq * (double)s->nc < kFltMinPairs) return f;
     std::vector<int32_t> len;
     for (auto &q : s->cls)
         if (!q.lanes) len.insert(len.end(), q.h_qlen.begin(), q.h_qlen.end());
@@ -1700,7 +1699,7 @@ static FilterPlan filter_plan(const blg_ctx *c, const blg_search *s, const SurvC
 static int search_run_bits(blg_ctx *c, blg_search *s, int dtype, void *d_out, bool *done) {
     *done = false;
     if (!s->tt || !s->bits_mem || bits_table_bytes(s->nsym, s->bits_longest) > kBitsMaxTable) return BLG_OK;
-    if (use_prefix(s) || !bits_faster(c, s)) return BLG_OK;
+    if (c->tuning || use_prefix(s) || !bits_faster(c, s)) return BLG_OK;
     BitSearch B{};
     B.Q = s->q.d;
     B.nq = s->bits_nq;
@@ -1755,7 +1754,7 @@ static int search_run(blg_ctx *c, blg_search *s, int k, int dtype, void *d_out, 
         const bool band = k <= 31 && C.n > 0;
         int64_t seq_q = 0;
         for (int i = 0; i < C.n; i++) seq_q += C.cls[i].nq;
-        const bool small = band && (double)seq_q * (double)s->nc <= kSmallPairs && seq_q <= 65535;
+        const bool small = band && !c->tuning && (double)seq_q * (double)s->nc <= kSmallPairs && seq_q <= 65535;
         if (small)
             CK(launch(c, "search_small", [&] {
                    return launch_search_small(c->stream, C, s->cs.d, s->perm, s->ccnt, s->qcnt, k, dtype, d_out, s->nc,
@@ -2034,7 +2033,6 @@ static void search_release(blg_ctx *c, blg_search *s) {
     s->sorted_mem = nullptr;
     s->perm = nullptr;
     s->lstart = nullptr;
-    s->csk = nullptr;
     s->lsorted = false;
     dev_free(c, s->tt_words);
     dev_free(c, s->tt_base);
@@ -2046,7 +2044,6 @@ static void search_release(blg_ctx *c, blg_search *s) {
     s->pfx = false;
     dev_free(c, s->sk_mem);
     s->sk_mem = nullptr;
-    s->csk = s->qsk = nullptr;
     s->csig = s->qsig = nullptr;
     s->ccnt = s->qcnt = nullptr;
     s->tt_words = nullptr;
@@ -2293,7 +2290,7 @@ static int batch_upload_body(blg_ctx *c, const blg_problem *pr, int nprob, blg_b
     }
     // ---- the meta block: B host-built tables, then C device-written
     struct At {
-        size_t hist = 0, tab = 0, perm = 0, soff = 0, csk = 0, ccnt = 0, sbuf = 0, qsk = 0, qcnt = 0;
+        size_t hist = 0, tab = 0, perm = 0, soff = 0, ccnt = 0, sbuf = 0, qcnt = 0;
         std::vector<size_t> both, lo, hi, wk, ts, peq;
     };
     std::vector<At> at((size_t)nprob);
@@ -2327,11 +2324,9 @@ static int batch_upload_body(blg_ctx *c, const blg_problem *pr, int nprob, blg_b
             at[i].tab = ml.take(sizeof(int64_t) * (size_t)(2 * n_len + 1));
             at[i].perm = ml.take(sizeof(int32_t) * (size_t)p.nc);
             at[i].soff = ml.take(sizeof(int64_t) * (size_t)(p.nc + 1));
-            at[i].csk = ml.take(sizeof(uint64_t) * (size_t)p.nc);
             at[i].ccnt = ml.take(sizeof(uint4) * (size_t)p.nc);
             at[i].sbuf = ml.take(kSlackBefore + (size_t)b->probs[i]->c.d.bytes + kSlackAfter) + kSlackBefore;
         }
-        at[i].qsk = ml.take(sizeof(uint64_t) * (size_t)p.nq);
         at[i].qcnt = ml.take(sizeof(uint4) * (size_t)p.nq);
         for (auto &q : prep[i].cls) {
             const size_t nq = q.idx.size();
@@ -2416,19 +2411,17 @@ static int batch_upload_body(blg_ctx *c, const blg_problem *pr, int nprob, blg_b
         s->q.d.n = p.nq;
         s->q.d.base = p.off_q[0];
         s->q.d.bytes = p.off_q[p.nq] - p.off_q[0];
-        s->qsk = (uint64_t *)(M + at[i].qsk);
         s->qcnt = (uint4 *)(M + at[i].qcnt);
         UploadPrep u{};                          // (the packed queries' slack came with the tables)
         u.buf[1] = (uint8_t *)s->c.d.buf;
         u.bytes[1] = s->c.d.bytes;
-        sks[nsk] = SketchSet{s->q.d, nullptr, nullptr, nullptr, s->qsk, s->qcnt, p.nq};
+        sks[nsk] = SketchSet{s->q.d, nullptr, nullptr, nullptr, s->qcnt, p.nq};
         sks_start[nsk + 1] = sks_start[nsk] + p.nq;
         nsk++;
         if (sorted[i]) {
             const int64_t n_len = P.mx - P.mn + 1;
             s->perm = (int32_t *)(M + at[i].perm);
             s->lstart = (int64_t *)(M + at[i].tab);
-            s->csk = (uint64_t *)(M + at[i].csk);
             s->ccnt = (uint4 *)(M + at[i].ccnt);
             s->cs.d.buf = M + at[i].sbuf;
             s->cs.d.off = (const int64_t *)(M + at[i].soff);
@@ -2450,7 +2443,7 @@ static int batch_upload_body(blg_ctx *c, const blg_problem *pr, int nprob, blg_b
             u.min_len = P.mn;
             u.n_sorted = p.nc;
             u.soff = (int64_t *)(M + at[i].soff);
-            sks[nsk] = SketchSet{s->c.d, s->perm, s->cs.d.off, M + at[i].sbuf, s->csk, s->ccnt, p.nc};
+            sks[nsk] = SketchSet{s->c.d, s->perm, s->cs.d.off, M + at[i].sbuf, s->ccnt, p.nc};
             sks_start[nsk + 1] = sks_start[nsk] + p.nc;
             nsk++;
         }
@@ -2500,8 +2493,6 @@ static int batch_upload_body(blg_ctx *c, const blg_problem *pr, int nprob, blg_b
             j.dtype = p.dtype;
             j.nw = cl.nw;
             j.tile = tile;
-            j.csk = s->csk;
-            j.qsk = s->qsk;
             j.ccnt = s->ccnt;
             j.qcnt = s->qcnt;
             j.out = p.d_out;
@@ -2638,7 +2629,10 @@ static int batch_run(blg_ctx *c, blg_batch *b) {
 //                        (timed at 24);
 //   short-pair tiles:    the staging shape (2^20 pairs of 32 bytes, 5%
 //                        edits, exact).
-// Results never depend on a shape; only time does.
+// Meanwhile the paths without a tuned shape that these inputs would take (the
+// bit-sliced search, the tensor-core filter, pairs by furthest-reaching points)
+// stand aside: the times would be theirs, the choice noise. Results never
+// depend on a shape; only time does.
 namespace {
 
 struct Rng {
@@ -3577,6 +3571,7 @@ int blg_autotune(blg_ctx *c, const char *cache_path) {
     if (cache_path && *cache_path && tuning_load(c, cache_path)) return BLG_OK;
     const int sched = c->sched;
     c->sched = BLG_SCHED_AUTO;
+    c->tuning = true;
     int rc = BLG_OK;
     for (int nw : {1, 2, 4})
         if (!rc) rc = tune_exact_search(c, nw);
@@ -3593,6 +3588,7 @@ int blg_autotune(blg_ctx *c, const char *cache_path) {
     if (!rc) rc = tune_band_pairs(c, 24);
     if (!rc) rc = tune_tile_pairs(c);
     c->sched = sched;
+    c->tuning = false;
     if (rc) {
         c->tune = blg_tuning();                         // keep the defaults on any failure
         return rc;

@@ -319,8 +319,7 @@ __global__ void __launch_bounds__(256) k_upload_prep(const UploadPrep *sets, con
 }
 
 // Every set's strings: the byte copy into sorted order (when the set has a
-// permutation), the 4-gram sketch and the binned 4-gram counts, a warp per
-// string. A warp takes 32 consecutive items; each lane first resolves one
+// permutation) and the binned 4-gram counts, a warp per string. A warp takes 32 consecutive items; each lane first resolves one
 // item (set, source string, destination) so the 32 lookups overlap, then
 // the warp walks the 32 strings, lane l taking the grams that start at
 // l, l + 32, .... A string of at most 256 bytes is read from shared memory,
@@ -328,21 +327,14 @@ __global__ void __launch_bounds__(256) k_upload_prep(const UploadPrep *sets, con
 // previous string; longer ones are read in place. Strings of at most 256
 // bytes have fewer than 256 grams, so the warp sums its byte counters with
 // plain adds; longer ones fold per-lane counters into saturating totals
-// every 255 grams and sum them with saturating byte adds. The sketch bits
-// are an OR over the warp.
-// Values equal gram_sketch / gram_counts of each string.
-__device__ __forceinline__ void gram_add(uint32_t g, int s, int n, uint32_t (&c)[4], uint32_t &sk_lo,
-                                         uint32_t &sk_hi) {
+// every 255 grams and sum them with saturating byte adds.
+// Values equal gram_counts of each string.
+__device__ __forceinline__ void gram_add(uint32_t g, int s, int n, uint32_t (&c)[4]) {
     if (s + 3 >= n) return;
     const uint32_t h = g * 0x9E3779B1u;
     const uint32_t bin = h >> 28, inc = 1u << (8 * (bin & 3));
 #pragma unroll
     for (int w = 0; w < 4; w++) c[w] += (bin >> 2) == (uint32_t)w ? inc : 0u;
-    if (s + 3 < kSketchWindow) {
-        const uint32_t bit = h >> 26;
-        if (bit < 32) sk_lo |= 1u << bit;
-        else sk_hi |= 1u << (bit - 32);
-    }
 }
 
 // Asynchronous 16-byte copies global -> shared (cp.async, no registers held
@@ -395,7 +387,6 @@ __global__ void __launch_bounds__(256) k_sketch_sets(const SketchSet *sets, cons
             }
             cp_async_commit();
         };
-        uint64_t my_sk = 0;
         uint4 my_cnt = make_uint4(0, 0, 0, 0);
         stage(0);
         for (int t = 0; t < cnt; t++) {
@@ -408,7 +399,6 @@ __global__ void __launch_bounds__(256) k_sketch_sets(const SketchSet *sets, cons
             uint8_t *q = reinterpret_cast<uint8_t *>(
                 __shfl_sync(kFull, (unsigned long long)reinterpret_cast<uintptr_t>(my_q), t));
             const int n = __shfl_sync(kFull, my_n, t);
-            uint32_t sk_lo = 0, sk_hi = 0;
             uint32_t tot[4] = {0, 0, 0, 0};                    // totals, bins 4w .. 4w+3
             if (n <= 256) {
                 // lane l takes positions 128c + 4l .. +3 of chunks c = 0, 1:
@@ -438,11 +428,6 @@ __global__ void __launch_bounds__(256) k_sketch_sets(const SketchSet *sets, cons
                                 const uint32_t one = 1u << (amt & 31u);
                                 if (amt & 32u) hi += one;
                                 else lo += one;
-                                if (c == 0 && sp + 3 < kSketchWindow) {
-                                    const uint32_t bit = h >> 26;
-                                    if (bit < 32) sk_lo |= 1u << bit;
-                                    else sk_hi |= 1u << (bit - 32);
-                                }
                             }
                             if (q && sp < n) q[sp] = (uint8_t)(a0 >> (8 * k));
                         }
@@ -468,7 +453,7 @@ __global__ void __launch_bounds__(256) k_sketch_sets(const SketchSet *sets, cons
                     const int c1 = min(n, c0 + 32 * 255);
                     for (int s = c0 + lane; s < c1; s += 32) {
                         const uint32_t w4 = load4(p + s);
-                        gram_add(__byte_perm(w4, 0u, 0x0123), s, n, c, sk_lo, sk_hi);
+                        gram_add(__byte_perm(w4, 0u, 0x0123), s, n, c);
                         if (q) q[s] = (uint8_t)w4;
                     }
 #pragma unroll
@@ -479,17 +464,11 @@ __global__ void __launch_bounds__(256) k_sketch_sets(const SketchSet *sets, cons
 #pragma unroll
                     for (int x = 0; x < 4; x++) tot[x] = __vaddus4(tot[x], __shfl_xor_sync(kFull, tot[x], off));
             }
-            sk_lo = __reduce_or_sync(kFull, sk_lo);
-            sk_hi = __reduce_or_sync(kFull, sk_hi);
-            if (lane == t) {
-                my_sk = ((uint64_t)sk_hi << 32) | sk_lo;
-                my_cnt = make_uint4(tot[0], tot[1], tot[2], tot[3]);
-            }
+            if (lane == t) my_cnt = make_uint4(tot[0], tot[1], tot[2], tot[3]);
             __syncwarp();                                      // buffer t & 1 is restaged for string t + 2
         }
         if (g0 + lane < total) {
             const SketchSet &S = sets[my_s];
-            S.sketch[my_i] = my_sk;
             S.counts[my_i] = my_cnt;
         }
     }

@@ -21,8 +21,6 @@ struct BatchJob {
     int64_t nc;
     int k, dtype, nw;
     int tile;                  // survivors per work unit: 4096 (banded survivor jobs) or 1024
-    const uint64_t *csk;       // 4-gram sketches of the sorted choices
-    const uint64_t *qsk;       // 4-gram sketches of the queries (by query row)
     const uint4 *ccnt;         // binned 4-gram counts of the sorted choices
     const uint4 *qcnt;         // binned 4-gram counts of the queries (by query row)
     void *out;
@@ -79,7 +77,6 @@ struct SketchSet {
     const int32_t *perm;
     const int64_t *dst_off;
     uint8_t *dst;
-    uint64_t *sketch;
     uint4 *counts;
     int64_t n;
 };

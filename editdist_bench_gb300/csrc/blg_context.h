@@ -48,6 +48,7 @@ struct blg_ctx {
     int sched = 0;                     // BLG_SCHED_* (work order of thresholded runs)
     blg_sched_model *model = nullptr;  // trained/loaded scheduler network, if any
     blg_tuning tune;                   // launch shapes (autotuned or defaults)
+    bool tuning = false;               // blg_autotune is timing: only kernels with a tuned shape run
     bool prof = false;
     // fault injection for tests of the error paths (blg_set_fault_injection):
     // the device allocation after `fault_alloc_after` more successes fails
