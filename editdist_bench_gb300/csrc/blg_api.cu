@@ -1918,18 +1918,32 @@ static int search_matches_rows(blg_ctx *c, blg_search *s, int k, int64_t q0, int
     return BLG_OK;
 }
 
-// LSD radix sort of list entries by their element index (entry >> 8), 8
-// bits per pass over the index bytes that vary.
+// LSD radix sort of list entries by their element index (entry >> 8), 11 bits
+// per pass over the index bits that vary, every pass counted in one read.
+// (32411 entries of 30 bits in the order in which the tensor-core filter's
+// passers were solved, which is none.)
 static void sort_by_index(std::vector<unsigned long long> &v) {
-    if (v.size() < 2) return;
+    if (v.size() < 512) {
+        std::sort(v.begin(), v.end());                   // indices are distinct
+        return;
+    }
+    constexpr int kBits = 11, kDigits = 1 << kBits;
     unsigned long long top = 0;
     for (auto e : v) top |= e >> 8;
+    int passes = 0;
+    while (passes * kBits < 56 && (top >> (passes * kBits)) != 0) passes++;
+    std::vector<uint32_t> cnt((size_t)passes * kDigits, 0);
+    for (auto e : v)
+        for (int p = 0; p < passes; p++) cnt[(size_t)p * kDigits + ((e >> (8 + p * kBits)) & (kDigits - 1))]++;
     std::vector<unsigned long long> tmp(v.size());
-    for (int shift = 8; shift < 64 && (top >> (shift - 8)) != 0; shift += 8) {
-        size_t cnt[257] = {0};
-        for (auto e : v) cnt[((e >> shift) & 0xffu) + 1]++;
-        for (int d = 0; d < 256; d++) cnt[d + 1] += cnt[d];
-        for (auto e : v) tmp[cnt[(e >> shift) & 0xffu]++] = e;
+    for (int p = 0; p < passes; p++) {
+        uint32_t *at = cnt.data() + (size_t)p * kDigits, sum = 0;
+        for (int d = 0; d < kDigits; d++) {
+            const uint32_t n = at[d];
+            at[d] = sum;
+            sum += n;
+        }
+        for (auto e : v) tmp[at[(e >> (8 + p * kBits)) & (kDigits - 1)]++] = e;
         v.swap(tmp);
     }
 }
@@ -1973,10 +1987,13 @@ static int search_matches_list(blg_ctx *c, blg_search *s, int k, blg_match *d_ou
                return launch_solve_passers(c->stream, c->sms, C, s->q.d, s->cs.d, s->perm, s->ccnt, s->qcnt, longest_query(s),
                                            k, BLG_UINT8, nullptr, s->nc, P, L, none, RepairPlan{}, c->d_status);
            }), "solve_passers");
-        CK(cudaMemcpyAsync(&passers, c->pl, sizeof(passers), cudaMemcpyDeviceToHost, c->stream), "D2H passers");
-        CK(cudaMemcpyAsync(&cnt, c->rl_hdr, sizeof(cnt), cudaMemcpyDeviceToHost, c->stream), "D2H list count");
+        // both counts beside each other in the lists' headers' spare words: one copy back
+        CK(cudaMemcpyAsync(c->pl + 1, c->rl_hdr, sizeof(cnt), cudaMemcpyDeviceToDevice, c->stream), "list count");
+        unsigned long long counts[2] = {0, 0};                     // passers, results
+        CK(cudaMemcpyAsync(counts, c->pl, sizeof(counts), cudaMemcpyDeviceToHost, c->stream), "D2H list counts");
         CK(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
-        listed = passers <= c->pl_cap;                             // else: the per-pair filter
+        cnt = counts[1];
+        listed = counts[0] <= c->pl_cap;                             // else: the per-pair filter
     }
     if (!listed) {
         const FillItems F{nullptr, nullptr, 0, BatchFill{nullptr, 0, BLG_UINT8, 0}, 0, c->rl_hdr + 1};
@@ -2008,10 +2025,12 @@ static int search_matches_list(blg_ctx *c, blg_search *s, int k, blg_match *d_ou
         staged.resize((size_t)m);
         rec = staged.data();
     }
+    int64_t q = 0;
     for (int64_t i = 0; i < m; i++) {
         const int64_t idx = (int64_t)(e[(size_t)i] >> 8);
-        rec[i].query = idx / s->nc;
-        rec[i].choice = idx % s->nc;
+        if (idx - q * s->nc >= s->nc) q = idx / s->nc;             // a division per row with matches
+        rec[i].query = q;
+        rec[i].choice = idx - q * s->nc;
         rec[i].dist = (int32_t)(e[(size_t)i] & 63u);
         rec[i].reserved = 0;
     }
