@@ -227,6 +227,7 @@ struct blg_search {
     uint16_t *tt_order = nullptr;     // per tile: positions by length, longest first
     int64_t max_len = 0;              // longest choice
     // exact runs, bit-sliced over the queries (k_search_bits): the distinct
+    int gram_sym = 256;              // the queries' bytes, as that many equally frequent ones (filter_plan)
     // bytes of the queries (nsym 0: not counted, or too many) and, per class set, the
     // sequential queries by length
     int nsym = 0;
@@ -1410,6 +1411,20 @@ static int search_run(blg_ctx *c, blg_search *s, int k, int dtype, void *d_out, 
 
 // Queries into HBM, with what `need` asks for: their 4-gram sketches
 // (thresholded runs), their symbols (exact runs).
+// As many equally frequent bytes as repeat as often as a sample's bytes do (DNA with
+// a rare N: 4), from up to 64 pieces of 64 bytes.
+static int sampled_symbols(const uint8_t *p, int64_t bytes) {
+    int64_t cnt[256] = {0}, n = 0;
+    const int64_t pieces = std::min<int64_t>(64, (bytes + 63) / 64);
+    for (int64_t i = 0; i < pieces; i++) {
+        const int64_t x0 = std::max<int64_t>(0, bytes - 64) * i / std::max<int64_t>(1, pieces - 1);
+        for (int64_t x = x0; x < std::min(bytes, x0 + 64); x++, n++) cnt[p[x]]++;
+    }
+    double same = 0.0;
+    for (int64_t v : cnt) same += (double)v * (double)v;
+    return n > 0 ? (int)((double)n * (double)n / same + 0.5) : 256;
+}
+
 static int search_upload_queries(blg_ctx *c, const uint8_t *bq, const int64_t *oq, int64_t nq, blg_search *s,
                                  unsigned need = NEED_ALL) {
     s->nq = nq;
@@ -1417,6 +1432,7 @@ static int search_upload_queries(blg_ctx *c, const uint8_t *bq, const int64_t *o
     if (rc) return rc;
     if ((need & NEED_TT) && nq > 0) query_symbols(bq, oq, nq, s);
     if (!(need & NEED_SORTED)) return BLG_OK;
+    if (nq > 0) s->gram_sym = sampled_symbols(bq + oq[0], oq[nq] - oq[0]);
     // one block: the signatures (32 B each), then the 4-gram counts (16 B each)
     const size_t nq1 = (size_t)std::max<int64_t>(nq, 1), o_cnt = sizeof(uint32_t) * kSigWords * nq1;
     CK(dev_alloc(c, &s->sk_mem, o_cnt + 16 * nq1), "cudaMallocAsync(sketches)");
@@ -1636,24 +1652,31 @@ struct FilterPlan {
     double filter_us = 0.0;
 };
 
-// The share of unrelated pairs of m-byte strings that pass at k, per length and
-// per number of bins from tables made once (a plan is part of every call).
+// The share of unrelated pairs of m-byte strings over nsym bytes that pass at k,
+// from tables made once (a plan is part of every call). nsym bytes have nsym^4
+// grams, which hash into so many of the bins: 256 of DNA into 160 of 248. (With all
+// 248 assumed, 1024 x 2^20 reads of 100 to 256 at max_dist 8 passed for a filter case and
+// ran the list full: 5.9 ms of matches against 5.2 without it.)
 struct PassShare {
-    static constexpr int kLen = 512, kSteps = 64;
-    float mean[2][kLen + 1], rsd[2][kLen + 1], tail[kSteps];
+    static constexpr int kLen = 512, kSteps = 64, kSym = 6;    // six bytes and more: all the bins
+    float mean[kSym][2][kLen + 1], rsd[kSym][2][kLen + 1], tail[kSteps];
     PassShare() {
-        const double bins[2] = {(double)kSigBins, (double)kSigBins / 2 - 4};
-        for (int h = 0; h < 2; h++)
-            for (int m = 0; m <= kLen; m++) {
-                const double p = 1.0 - std::exp(-std::max(0, m - 3) / bins[h]), x = 2.0 * p * (1.0 - p);
-                mean[h][m] = (float)(x * bins[h]);
-                rsd[h][m] = (float)(1.0 / std::sqrt(std::max(1.0, bins[h] * x * (1.0 - x))));
+        for (int a = 0; a < kSym; a++)
+            for (int h = 0; h < 2; h++) {
+                const double all = h ? (double)kSigBins / 2 - 4 : (double)kSigBins, grams = std::pow(a + 1.0, 4.0);
+                const double bins = all * (1.0 - std::exp(-grams / all));
+                for (int m = 0; m <= kLen; m++) {
+                    const double p = 1.0 - std::exp(-std::max(0, m - 3) / bins), x = 2.0 * p * (1.0 - p);
+                    mean[a][h][m] = (float)(x * bins);
+                    rsd[a][h][m] = (float)(1.0 / std::sqrt(std::max(1.0, bins * x * (1.0 - x))));
+                }
             }
         for (int i = 0; i < kSteps; i++) tail[i] = (float)(0.5 * std::erfc(i / 8.0 / 1.41421356));   // beyond i / 8 deviations
     }
-    double operator()(int m, int half, int k) const {
+    double operator()(int m, int half, int k, int nsym) const {
+        const int a = std::max(1, std::min(nsym, (int)kSym)) - 1;
         m = std::min(m, kLen);
-        const float z = (mean[half][m] - 8.0f * (float)k) * rsd[half][m];
+        const float z = (mean[a][half][m] - 8.0f * (float)k) * rsd[a][half][m];
         if (z <= 0.0f) return 1.0 - tail[std::min(kSteps - 1, (int)(-z * 8.0f))];
         return tail[std::min(kSteps - 1, (int)(z * 8.0f))];
     }
@@ -1681,8 +1704,8 @@ static FilterPlan filter_plan(const blg_ctx *c, const blg_search *s, const SurvC
             while (e < q1 && len[e] == len[q]) e++;
             const double n = (double)(e - q) * (double)window(len[q], len[q]);
             pairs += n;
-            pass += n * pass_share(len[q], 0, k);
-            pass_folded += n * pass_share(len[q], 1, k);
+            pass += n * pass_share(len[q], 0, k, s->gram_sym);
+            pass_folded += n * pass_share(len[q], 1, k, s->gram_sym);
             q = e;
         }
         tiles += std::ceil((double)window(len[q0], len[q1 - 1]) / 256.0);
@@ -1977,7 +2000,6 @@ static int search_matches_list(blg_ctx *c, blg_search *s, int k, blg_match *d_ou
     if (fp.pays) {
         const PasserList P{c->pl + 4, c->pl, c->pl_cap};
         const BatchFill none{nullptr, 0, BLG_UINT8, 0};
-        unsigned long long passers = 0;
         CK(cudaMemsetAsync(c->pl, 0, 4 * sizeof(unsigned long long), c->stream), "clear list");
         CK(launch(c, "filter_pairs", [&] {
                return launch_filter_pairs(c->stream, c->sms, C, fp.nq, s->qsig, s->csig, fp.folded, s->lstart, s->min_len,

@@ -59,7 +59,7 @@ def _sets(rng, nq, nc, lo, hi, alphabet, rate=0.06):
 @pytest.mark.gpu
 @pytest.mark.parametrize("nq,nc,lo,hi,alphabet,k", [(128, 32768, 64, 64, "dna", 2), (900, 5001, 64, 64, "dna", 0),
                                                     (257, 20003, 50, 80, "dna", 4), (1000, 20001, 100, 140, "dna", 3),
-                                                    (260, 16001, 172, 172, "dna", 13), (129, 32001, 18, 18, "text", 1),
+                                                    (260, 16001, 172, 172, "text", 13), (129, 32001, 18, 18, "text", 1),
                                                     (600, 30011, 20, 60, "text", 2)])
 def test_filter_search(gpu, nq, nc, lo, hi, alphabet, k):
     rng = np.random.default_rng(nq + nc + k)
