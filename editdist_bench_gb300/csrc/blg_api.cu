@@ -226,8 +226,8 @@ struct blg_search {
     int32_t *tt_len = nullptr;
     uint16_t *tt_order = nullptr;     // per tile: positions by length, longest first
     int64_t max_len = 0;              // longest choice
-    // exact runs, bit-sliced over the queries (k_search_bits): the distinct
     int gram_sym = 256;              // the queries' bytes, as that many equally frequent ones (filter_plan)
+    // exact runs, bit-sliced over the queries (k_search_bits): the distinct
     // bytes of the queries (nsym 0: not counted, or too many) and, per class set, the
     // sequential queries by length
     int nsym = 0;
@@ -1409,8 +1409,6 @@ static int search_upload_choices(blg_ctx *c, const uint8_t *bc, const int64_t *o
 static int search_run(blg_ctx *c, blg_search *s, int k, int dtype, void *d_out, int64_t q0 = 0,
                       int64_t q1 = -1);
 
-// Queries into HBM, with what `need` asks for: their 4-gram sketches
-// (thresholded runs), their symbols (exact runs).
 // As many equally frequent bytes as repeat as often as a sample's bytes do (DNA with
 // a rare N: 4), from up to 64 pieces of 64 bytes.
 static int sampled_symbols(const uint8_t *p, int64_t bytes) {
@@ -1425,6 +1423,8 @@ static int sampled_symbols(const uint8_t *p, int64_t bytes) {
     return n > 0 ? (int)((double)n * (double)n / same + 0.5) : 256;
 }
 
+// Queries into HBM, with what `need` asks for: their 4-gram counts and signatures
+// (thresholded runs), their symbols (exact runs).
 static int search_upload_queries(blg_ctx *c, const uint8_t *bq, const int64_t *oq, int64_t nq, blg_search *s,
                                  unsigned need = NEED_ALL) {
     s->nq = nq;
