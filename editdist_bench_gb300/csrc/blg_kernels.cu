@@ -20,9 +20,12 @@
 //                       pattern exceeds 64 go to a device queue.
 //  * k_pairs_long       persistent consumer of that queue, lane-spread.
 //  * k_search_surv      thresholded cdist with max_dist > 31 (full-word loop);
-//                       max_dist <= 31 runs in blg_search_lpt.cu.
+//                       max_dist <= 31 runs in blg_search_band.cu and, where
+//                       its 4-gram filter is a matrix product worth making,
+//                       blg_search_filter.cu; exact cdist mostly in
+//                       blg_search_bits.cu.
 //
-// All arithmetic is integer bit logic on the ALU/FMA pipes; no tensor cores.
+// All arithmetic here is integer bit logic on the ALU/FMA pipes.
 #include <algorithm>
 
 #include "blg_kernels.cuh"
