@@ -1644,8 +1644,13 @@ static bool bits_faster(const blg_ctx *c, const blg_search *s) {
 // grams a string fills p = 1 - exp(-g / bins) of its bins and two unrelated
 // strings differ in 2 p (1 - p) of them, give or take the binomial
 // deviation; the share below 8 k passes to the list, which has to stay well
-// within its room. Half the bins where that lets hardly more through: half the
-// product and half the rows to write.
+// within its room (an eighth of it: max_dist 6 on 1024 x 2^18 reads of 100 to 256
+// 262 us, 385 per pair; at all of it max_dist 7 ran the list full, 919 and 765) and
+// a small part of the pairs (257 x 100003 lines of 20 to 120 at max_dist 6, one in
+// ten: 119 us, 91 per pair). Half the bins where that lets no more through: half
+// the product and half the rows to write, which the warps that read the
+// sums hide; 13 thousand more passers cost far more (1024 x 2^18 reads of 64 at
+// max_dist 4: 246 us folded, 90 whole).
 struct FilterPlan {
     bool pays = false, folded = false;
     int nq = 0;
@@ -1711,9 +1716,9 @@ static FilterPlan filter_plan(const blg_ctx *c, const blg_search *s, const SurvC
         tiles += std::ceil((double)window(len[q0], len[q1 - 1]) / 256.0);
     }
     f.nq = (int)nq;
-    f.folded = pass_folded <= pass + 1e-4 * pairs;
+    f.folded = pass_folded <= pass + 1e-7 * pairs;
     f.filter_us = 6.0 + std::ceil(tiles / c->sms) * (f.folded ? 0.75 : 1.15);
-    f.pays = pairs >= 1800.0 * tiles && pairs >= kFltMinPairs && pass <= (double)c->pl_cap / 16.0;
+    f.pays = pairs >= 1800.0 * tiles && pairs >= kFltMinPairs && pass <= std::min((double)c->pl_cap / 8.0, pairs / 32.0);
     return f;
 }
 
