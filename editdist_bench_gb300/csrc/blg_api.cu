@@ -1803,7 +1803,7 @@ static int search_run(blg_ctx *c, blg_search *s, int k, int dtype, void *d_out, 
             if (!whole_fill) CK(cudaMemsetAsync(c->rl_hdr, 0, sizeof(unsigned long long), c->stream), "clear list");
             CK(launch(c, "filter_pairs", [&] {
                    return launch_filter_pairs(c->stream, c->sms, C, fp.nq, s->qsig, s->csig, fp.folded, s->lstart, s->min_len,
-                                              s->n_len, k, P, whole, whole_fill, c->d_status);
+                                              s->n_len, k, P, whole, whole_fill, c->fault_wait_polls, c->d_status);
                }), "filter_pairs");
             CK(launch(c, "solve_passers", [&] {
                    return launch_solve_passers(c->stream, c->sms, C, s->q.d, s->cs.d, s->perm, s->ccnt, s->qcnt,
@@ -2008,7 +2008,7 @@ static int search_matches_list(blg_ctx *c, blg_search *s, int k, blg_match *d_ou
         CK(cudaMemsetAsync(c->pl, 0, 4 * sizeof(unsigned long long), c->stream), "clear list");
         CK(launch(c, "filter_pairs", [&] {
                return launch_filter_pairs(c->stream, c->sms, C, fp.nq, s->qsig, s->csig, fp.folded, s->lstart, s->min_len,
-                                          s->n_len, k, P, none, true, c->d_status);
+                                          s->n_len, k, P, none, true, c->fault_wait_polls, c->d_status);
            }), "filter_pairs");
         CK(launch(c, "solve_passers", [&] {
                return launch_solve_passers(c->stream, c->sms, C, s->q.d, s->cs.d, s->perm, s->ccnt, s->qcnt, longest_query(s),

@@ -115,15 +115,23 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 }
 
 // A role's wait: bounded; one that gives up raises the status bit and the
-// CTA's abort flag, on which every role leaves its loop.
-__device__ __forceinline__ bool role_wait(int *abort, uint64_t *bar, uint32_t parity, uint32_t *status) {
-    for (uint32_t i = 0; i < kMbarPolls; i++) {
+// CTA's abort flag, on which every role leaves its loop. A lane's own verdict:
+// for the lane that issues the products alone.
+__device__ __forceinline__ bool role_wait(int *abort, uint64_t *bar, uint32_t parity, uint32_t polls, uint32_t *status) {
+    for (uint32_t i = 0; i < polls; i++) {
         if (mbar_try_wait(bar, parity)) return true;
         if (*(volatile int *)abort) return false;
     }
     atomicOr(status, ST_QUEUE_TIMEOUT);
     *(volatile int *)abort = 1;
     return false;
+}
+
+// The wait of a whole warp, one verdict for all lanes: near the bound, or with
+// the flag just raised, lanes see different things, and what follows in the
+// reading and producing warps (TMEM loads, votes, shuffles) needs all of them.
+__device__ __forceinline__ bool warp_wait(int *abort, uint64_t *bar, uint32_t parity, uint32_t polls, uint32_t *status) {
+    return __all_sync(kFull, role_wait(abort, bar, parity, polls, status));
 }
 
 // The output's k + 1, in items of kFillItem bytes from its first 16-byte
@@ -198,7 +206,7 @@ __device__ __forceinline__ void write_row(uint8_t *dst, int r, int j0, int j1, W
 template <int K>
 __global__ void __launch_bounds__(kFltThreads, 1)
     k_filter_pairs(SurvClasses C, int nq, const uint32_t *qsig, const uint32_t *csig, const int64_t *lstart,
-                   int64_t min_len, int64_t n_len, int k, PasserList L, BatchFill fill, bool whole_fill,
+                   int64_t min_len, int64_t n_len, int k, PasserList L, BatchFill fill, bool whole_fill, uint32_t polls,
                    uint32_t *status) {
     extern __shared__ __align__(128) uint8_t s_raw[];
     FilterShared<K> &S = *reinterpret_cast<FilterShared<K> *>(s_raw);
@@ -281,8 +289,8 @@ __global__ void __launch_bounds__(kFltThreads, 1)
             for (int i = 0; i < ntiles; i++) {
                 const int buf = i & 1;
                 const uint32_t par = (uint32_t)(i >> 1) & 1u;
-                if (!role_wait(&S.abort, &S.full[buf], par, status)) break;
-                if (!role_wait(&S.abort, &S.tempty[buf], par ^ 1u, status)) break;
+                if (!role_wait(&S.abort, &S.full[buf], par, polls, status)) break;
+                if (!role_wait(&S.abort, &S.tempty[buf], par ^ 1u, polls, status)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t a = smem_addr(S.a), b = smem_addr(S.b[buf]);
 #pragma unroll
@@ -343,7 +351,7 @@ __global__ void __launch_bounds__(kFltThreads, 1)
         };
         for (int i = 0; i < ntiles; i++) {
             const int buf = i & 1;
-            if (!role_wait(&S.abort, &S.tfull[buf], (uint32_t)(i >> 1) & 1u, status)) break;
+            if (!warp_wait(&S.abort, &S.tfull[buf], (uint32_t)(i >> 1) & 1u, polls, status)) break;
             advance(i);
             __syncwarp();
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -392,10 +400,10 @@ __global__ void __launch_bounds__(kFltThreads, 1)
             if (K == 128) sig_fold(wd);
             const bool valid = nvalid;
             if (i + 1 < ntiles) fetch(i + 1);
-            if (!role_wait(&S.abort, &S.empty[buf], par ^ 1u, status)) break;
+            if (!warp_wait(&S.abort, &S.empty[buf], par ^ 1u, polls, status)) break;
             if (qcur != built) {
                 // the queries' rows: every product on the old ones has to be done
-                if (i > 0 && !role_wait(&S.abort, &S.empty[buf ^ 1], (uint32_t)((i - 1) >> 1) & 1u, status)) break;
+                if (i > 0 && !warp_wait(&S.abort, &S.empty[buf ^ 1], (uint32_t)((i - 1) >> 1) & 1u, polls, status)) break;
                 built = qcur;
                 const int row = r & (kFltM - 1), half = r / kFltM;       // two threads a row
                 const int q = qcur * kFltM + row;
@@ -431,8 +439,10 @@ __global__ void __launch_bounds__(kFltThreads, 1)
         }
     }
     }
-    // products in flight end before TMEM goes back: the last commits of both buffers
-    for (int i = max(0, issued - 2); i < issued; i++) mbar_wait(&S.tfull[i & 1], (uint32_t)(i >> 1) & 1u);
+    // products in flight end before TMEM goes back: the last commits of both
+    // buffers (under the normal bound, whatever `polls` is)
+    for (int i = max(0, issued - 2); i < issued; i++)
+        if (!mbar_wait(&S.tfull[i & 1], (uint32_t)(i >> 1) & 1u)) atomicOr(status, ST_QUEUE_TIMEOUT);
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -564,23 +574,25 @@ __global__ void __launch_bounds__(256)
 template <int K>
 static cudaError_t launch_filter_k(cudaStream_t st, int sms, const SurvClasses &C, int nq, const uint32_t *qsig,
                                    const uint32_t *csig, const int64_t *lstart, int64_t min_len, int64_t n_len, int k,
-                                   const PasserList &L, const BatchFill &fill, bool whole_fill, uint32_t *status) {
+                                   const PasserList &L, const BatchFill &fill, bool whole_fill, uint32_t polls,
+                                   uint32_t *status) {
     const int smem = (int)sizeof(FilterShared<K>);
     const cudaError_t e = cudaFuncSetAttribute(k_filter_pairs<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     k_filter_pairs<K><<<sms, kFltThreads, smem, st>>>(C, nq, qsig, csig, lstart, min_len, n_len, k, L, fill, whole_fill,
-                                                      status);
+                                                      polls, status);
     return cudaGetLastError();
 }
 
 cudaError_t launch_filter_pairs(cudaStream_t st, int sms, const SurvClasses &C, int nq, const uint32_t *qsig,
                                 const uint32_t *csig, bool folded, const int64_t *lstart, int64_t min_len,
                                 int64_t n_len, int k, const PasserList &L, const BatchFill &fill, bool whole_fill,
-                                uint32_t *status) {
+                                int32_t wait_polls, uint32_t *status) {
     if (nq <= 0 || C.n <= 0) return cudaSuccess;
     if (k < 0 || k > kSigMaxK || (nq + kFltM - 1) / kFltM > kFltMaxTiles) return cudaErrorInvalidValue;
-    return folded ? launch_filter_k<128>(st, sms, C, nq, qsig, csig, lstart, min_len, n_len, k, L, fill, whole_fill, status)
-                  : launch_filter_k<256>(st, sms, C, nq, qsig, csig, lstart, min_len, n_len, k, L, fill, whole_fill, status);
+    const uint32_t polls = wait_polls < 0 ? kMbarPolls : (uint32_t)wait_polls;
+    return folded ? launch_filter_k<128>(st, sms, C, nq, qsig, csig, lstart, min_len, n_len, k, L, fill, whole_fill, polls, status)
+                  : launch_filter_k<256>(st, sms, C, nq, qsig, csig, lstart, min_len, n_len, k, L, fill, whole_fill, polls, status);
 }
 
 cudaError_t launch_solve_passers(cudaStream_t st, int sms, const SurvClasses &C, const DevStrings &Q,

@@ -29,10 +29,12 @@ struct RepairPlan {
 
 // fill: the output to set to k + 1 (n = 0: none); whole_fill: by the filter
 // alone, else the solver goes on with it. folded: signatures of half the bins.
+// wait_polls: the roles' waits on one another give up after that many polls (-1:
+// the normal bound); a run that did raises ST_QUEUE_TIMEOUT.
 cudaError_t launch_filter_pairs(cudaStream_t st, int sms, const SurvClasses &C, int nq, const uint32_t *qsig,
                                 const uint32_t *csig, bool folded, const int64_t *lstart, int64_t min_len,
                                 int64_t n_len, int k, const PasserList &L, const BatchFill &fill, bool whole_fill,
-                                uint32_t *status);
+                                int32_t wait_polls, uint32_t *status);
 // Results <= k into `out` (L.item null) or into L. longest: of the queries.
 cudaError_t launch_solve_passers(cudaStream_t st, int sms, const SurvClasses &C, const DevStrings &Q,
                                  const DevStrings &CS, const int32_t *perm, const uint4 *ccnt, const uint4 *qcnt,

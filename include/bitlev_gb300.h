@@ -270,9 +270,10 @@ int blg_synchronize(blg_ctx *ctx);
  * allocations of this context succeed, the next one fails as if the device
  * were out of memory (BLG_ERR_ALLOC); the hook is then spent. -1: off.
  * wait_polls >= 0: the short-pair tile kernel's bounded wait for its staged
- * strings gives up after that many polls instead of its normal bound, so the
- * call ends with BLG_ERR_TIMEOUT (the kernel still waits, at the normal
- * bound, for its copies in flight before it returns). -1: normal bound.
+ * strings, and the waits of the thresholded search's tensor-core filter, give
+ * up after that many polls instead of their normal bound, so the call ends
+ * with BLG_ERR_TIMEOUT (the kernels still wait, at the normal bound, for their
+ * copies and products in flight before they return). -1: normal bound.
  * Nothing here faults, traps or hangs the GPU; the context stays usable. */
 int blg_set_fault_injection(blg_ctx *ctx, int64_t alloc_fail_after, int32_t wait_polls);
 
