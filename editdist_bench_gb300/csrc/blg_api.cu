@@ -14,6 +14,7 @@
 #include <cmath>
 #include <condition_variable>
 #include <functional>
+#include <numeric>
 #include <thread>
 #include <cstdio>
 #include <cstdlib>
@@ -122,8 +123,9 @@ constexpr size_t kBitsMaxTable = 160 << 10;
 constexpr size_t kBitsMaxScratch = size_t(512) << 20;
 // The prefix-reuse kernel where the restarts skip enough of the text (it takes
 // 16.3 ms on 4096 x 65536 reads of 64 bases with none skipped, the bit-sliced
-// one 9.2), and for 33 to 64 queries, where its tests hold it to that path
-// (64 x 20000 reads of 64: 186 us against 77).
+// one 9.2). Searches of 33 to 64 queries of at most two words take it too,
+// which is the slower side (64 x 20000 reads of 64: 186 us against 77; 64 x
+// 65536: 498 against 183): tests/test_gpu_prefix.py expects this kernel there.
 constexpr double kBitsPfxSaving = 0.45;
 constexpr int kPfxMinQueries = 33, kPfxMaxQueries = 64;
 // Tensor-core filter: pairs below which its launch costs more than it saves.
@@ -226,6 +228,7 @@ struct blg_search {
     int32_t *tt_len = nullptr;
     uint16_t *tt_order = nullptr;     // per tile: positions by length, longest first
     int64_t max_len = 0;              // longest choice
+    double warp_len = 0.0;            // mean of the longest of 32 neighbours
     int gram_sym = 256;              // the queries' bytes, as that many equally frequent ones (filter_plan)
     // exact runs, bit-sliced over the queries (k_search_bits): the distinct
     // bytes of the queries (nsym 0: not counted, or too many) and, per class set, the
@@ -234,6 +237,7 @@ struct blg_search {
     uint8_t sym_map[256];
     void *bits_mem = nullptr;         // [group weights | qidx | qlen] of the sequential queries
     int bits_nq = 0, bits_longest = 0;
+    double bits_share = 1.0;          // mean weight of its groups over the heaviest's
 };
 
 // ------------------------------------------------------------ helpers --
@@ -1032,6 +1036,8 @@ static int bits_build(blg_ctx *c, const std::vector<QueryClass> &qc, blg_search 
     CK(cudaMemcpyAsync(s->bits_mem, host.data(), 8 * host.size(), cudaMemcpyHostToDevice, c->stream), "H2D queries");
     s->bits_nq = (int)nq;
     s->bits_longest = len.back();
+    const int64_t first = host[1];                          // the group of the longest
+    s->bits_share = first > 0 ? (double)host[groups] / ((double)first * (double)groups) : 1.0;
     return BLG_OK;                                       // (pageable: the copy completed before return)
 }
 
@@ -1367,17 +1373,23 @@ static int search_upload_choices(blg_ctx *c, const uint8_t *bc, const int64_t *o
         std::vector<int64_t> base(tiles + 1, 0);
         HostPool &pool = HostPool::get();
         const int nt = nc >= (1 << 16) ? pool.size() : 1;
-        std::vector<int64_t> longest((size_t)nt, 0);
-        pool.run(nt, [&](int w) {                               // each tile's longest choice
+        std::vector<int64_t> longest((size_t)nt, 0), by_warp((size_t)nt, 0);
+        pool.run(nt, [&](int w) {                               // each tile's longest choice, and each warp's
             for (int64_t t = tiles * w / nt, te = tiles * (w + 1) / nt; t < te; t++) {
                 int64_t mx = 0;
                 const int64_t e = std::min(nc, (t + 1) * kTileCands);
-                for (int64_t i = t * kTileCands; i < e; i++) mx = std::max(mx, oc[i + 1] - oc[i]);
+                for (int64_t i0 = t * kTileCands; i0 < e; i0 += 32) {
+                    int64_t wm = 0;
+                    for (int64_t i = i0; i < std::min(e, i0 + 32); i++) wm = std::max(wm, oc[i + 1] - oc[i]);
+                    by_warp[w] += wm;
+                    mx = std::max(mx, wm);
+                }
                 base[t + 1] = kTileCands * ((mx + 3) / 4);
                 longest[w] = std::max(longest[w], mx);
             }
         });
         s->max_len = *std::max_element(longest.begin(), longest.end());
+        s->warp_len = (double)std::accumulate(by_warp.begin(), by_warp.end(), (int64_t)0) / (double)((nc + 31) / 32);
         for (int64_t t = 0; t < tiles; t++) base[t + 1] += base[t];
         const int64_t bytes = oc[nc] - oc[0];
         if (base[tiles] * 4 <= 2 * bytes + (64ll << 20)) {
@@ -1408,6 +1420,7 @@ static int search_upload_choices(blg_ctx *c, const uint8_t *bc, const int64_t *o
 
 static int search_run(blg_ctx *c, blg_search *s, int k, int dtype, void *d_out, int64_t q0 = 0,
                       int64_t q1 = -1);
+static bool bits_applies(blg_ctx *c, const blg_search *s);
 
 // As many equally frequent bytes as repeat as often as a sample's bytes do (DNA with
 // a rare N: 4), from up to 64 pieces of 64 bytes.
@@ -1499,10 +1512,9 @@ static int cdist_pipelined(blg_ctx *c, const uint8_t *bq, const int64_t *oq, int
             // exact runs: the host sorts the choices for the prefix-reuse
             // kernel while the first chunk computes on the tile-transposed
             // copy; the later chunks use it
-            // (only where the bit-sliced kernel would not beat it)
+            // (only where the bit-sliced kernel cannot run or would not beat it)
             if (!rc && ch == 0 && k < 0 && nch > 1 &&
-                ((s->bits_nq >= kPfxMinQueries && s->bits_nq <= kPfxMaxQueries) || s->bits_nq == 0 ||
-                 sampled_prefix_share(bc, oc, nc) >= 0.7 * kBitsPfxSaving))
+                (!bits_applies(c, s) || sampled_prefix_share(bc, oc, nc) >= 0.7 * kBitsPfxSaving))
                 rc = search_build_prefix(c, bc, oc, nc, s);
             if (rc) break;
         }
@@ -1603,36 +1615,74 @@ static int64_t class_queries(const blg_search *s) {
 }
 
 // Whether the exact run of the sequential classes takes the prefix-reuse kernel
-// for its one- and two-word classes.
+// for its one- and two-word classes whatever the others' estimates. A chunk of a
+// larger search (cdist_pipelined) is no search of 33 to 64 queries.
 static bool use_prefix(const blg_search *s) {
-    return s->pfx && ((s->bits_nq >= kPfxMinQueries && s->bits_nq <= kPfxMaxQueries) ||
-                      s->pfx_saving >= kBitsPfxSaving || s->bits_nq == 0);
+    const bool held = s->bits_nq >= kPfxMinQueries && s->bits_nq <= kPfxMaxQueries && s->bits_longest <= 128 &&
+                      class_queries(s) == s->nq;
+    return s->pfx && (held || s->pfx_saving >= kBitsPfxSaving || s->bits_nq == 0);
 }
 
-// Whether the bit-sliced kernel beats the per-class word kernels on an exact
-// run. Both have a floor, the time a lone warp takes for its longest strings,
-// and a rate. Measured (GB300, 1 to 256 queries x 200 to 60000 choices of 12
-// to 256 bytes; microseconds bit-sliced / word): a bit-sliced unit takes 6.6
-// ns per cell of its 32 x 32 pairs alone and four fifths of that when an SM
-// partition has several; a word kernel's thread 37 ns per column and word
-// (four words at least: short queries go four at a time), for up to four
-// choices one after the other, and 1.12 ps per column and word at full rate.
-// 64 x 64 bytes: 32 x 200 34 / 13, 1 x 2000 32 / 42, 32 x 60000 93 / 483;
-// 256 x 256 bytes: 32 x 3500 389 / 169, 32 x 20000 654 / 820, 256 x 60000
-// 8414 / 17565.
-static bool bits_faster(const blg_ctx *c, const blg_search *s) {
+// Estimated microseconds of an exact run, by kernel: each has a floor, the time of
+// its longest strings, and a rate. Fitted to 1 to 1000 queries x 100 to 65536
+// choices of 5 to 512 bytes (GB300, DNA).
+// The word kernels (k_search_tt) give a thread up to four choices, one after the
+// other, and take the queries of one or two words four or two at a time, real or
+// not: a block of pick_qpb's 1 query costs what one of 4 does. Few blocks go by
+// whole rounds over the SMs. 32 x 20000 reads of 64: 195 (206 measured, 44 if only
+// real queries counted); 16 x 20000: 119 (128); 500 x 5000: 370 (357).
+static double word_us(blg_ctx *c, const blg_search *s, const blg_search::Cls &k) {
+    const int64_t nc = s->nc, qpb = pick_qpb(c, k.nw, k.nq, nc), qi = k.nw == 1 ? 4 : k.nw == 2 ? 2 : 1;
+    auto slots = [&](int64_t q) { return (q + qi - 1) / qi * qi; };
+    const double cols = (double)s->max_len, pairs = (double)(k.nq / qpb * slots(qpb) + slots(k.nq % qpb)) * (double)((nc + 31) & ~int64_t(31));
+    const double floor = 37e-3 * cols * std::max(4, k.nw) * (double)std::min<int64_t>(4, (nc + 255) / 256) * (double)(slots(qpb) / qi);
+    const int64_t blocks = (nc + kTileCands - 1) / kTileCands * ((k.nq + qpb - 1) / qpb), rounds = (blocks + c->sms - 1) / c->sms;
+    return 5.0 + std::max(floor * (double)(rounds <= 4 ? rounds : 1), 1.12e-6 * s->warp_len * k.nw * pairs);
+}
+
+// The prefix-reuse kernel's lanes hold queries, 128 of one word or 64 of two to a
+// warp, real or not. 500 x 20000 reads of 64: 668 (621 measured); 1 x 20000: 206 (185).
+static double prefix_us(const blg_search *s, const blg_search::Cls &k) {
+    const double cols = (double)s->max_len, avg = (double)s->c.d.bytes / (double)s->nc, slots = k.nw == 1 ? 128.0 : 64.0;
+    const double rate = 1.1e-6 * (1.0 - s->pfx_saving) * avg * k.nw * std::ceil(k.nq / slots) * slots * (double)s->nc;
+    return 5.0 + std::max(1.6 * cols, 0.6 * cols + rate);
+}
+
+// Whether a class that is not bit-sliced takes the prefix-reuse kernel: where its
+// layout was built, unless the word kernel is well ahead (1 x 65536 reads of 16 to
+// 256: 157 against 1180; 100 x 5000 reads of 64: 165 against 104).
+static bool class_prefix(blg_ctx *c, const blg_search *s, const blg_search::Cls &k) {
+    if (!s->pfx || !search_pfx_supported(k.nw)) return false;
+    return use_prefix(s) || c->tuning || word_us(c, s, k) >= 0.8 * prefix_us(s, k);
+}
+
+// Whether the bit-sliced kernel beats the others on an exact run. A unit takes 6.6
+// ns per cell of its 32 x 32 pairs alone on its SM partition and 1.6 times that with
+// a second one beside it, two rounds over the eight warps of an SM cost twice, and a
+// CTA with units of two groups waits for the last of the first. Before the last
+// round, shorter choices and groups count as such. 33 x 65536 reads of 256: 2.7 ms
+// (2.8 measured, 2.3 of the word kernel); 4 x 40000 of 16 to 256: 0.81 (0.85, 0.51);
+// 32 x 20000 of 64: 51 us (52, 206); 1000 x 20000: 735 (767, 1386).
+static bool bits_faster(blg_ctx *c, const blg_search *s) {
     const double cols = (double)s->max_len, avg = (double)s->c.d.bytes / (double)s->nc;
-    const double units = (double)((s->bits_nq + 31) / 32) * (double)((s->nc + 31) / 32);
+    const int64_t groups = (s->bits_nq + 31) / 32, units = groups * ((s->nc + 31) / 32), slots = bits_warps(c->sms);
     const double alone = 6.6e-3 * cols * (double)std::max(8, (s->bits_longest + 7) & ~7);
-    const double waves = std::ceil(units / (4.0 * c->sms));
-    const double bits = 8.0 + alone * std::max(1.0, 0.8 * waves * (waves > 2 ? avg / std::max(cols, 1.0) : 1.0));
-    double word = 0.0;
-    for (auto &k : s->cls) {
-        if (k.lanes) continue;
-        const double floor = 37e-3 * cols * std::max(4, k.nw) * (double)std::min<int64_t>(4, (s->nc + 255) / 256);
-        word += 5.0 + std::max(floor, 1.12e-6 * avg * k.nw * (double)k.nq * (double)s->nc);
-    }
-    return bits <= word;
+    const double full = (double)(units / slots), rem = (double)(units % slots);
+    double rounds = 1.6 * full * (cols > 0.0 ? avg / cols : 1.0) * s->bits_share;
+    rounds += rem == 0.0 ? 0.0 : 2.0 * rem <= (double)slots ? 1.0 : 1.6;
+    if (groups > 1 && full > 0.0) rounds += 0.3;
+    const double bits = 8.0 + alone * std::max(1.0, rounds);
+    double other = 0.0;
+    for (auto &k : s->cls)
+        if (!k.lanes) other += class_prefix(c, s, k) ? prefix_us(s, k) : word_us(c, s, k);
+    return bits <= 1.05 * other;
+}
+
+// Whether the bit-sliced kernel can run, and is the faster one, on the current classes.
+static bool bits_applies(blg_ctx *c, const blg_search *s) {
+    if (!s->tt || !s->bits_mem || c->tuning || bits_table_bytes(s->nsym, s->bits_longest) > kBitsMaxTable) return false;
+    const size_t scratch = s->bits_longest > 64 ? sizeof(uint32_t) * (size_t)bits_scratch_words(s->max_len) * (size_t)bits_warps(c->sms) : 0;
+    return scratch <= kBitsMaxScratch && bits_faster(c, s);
 }
 
 // Whether a thresholded run of the sequential classes filters on the tensor
@@ -1726,8 +1776,7 @@ static FilterPlan filter_plan(const blg_ctx *c, const blg_search *s, const SurvC
 // *done = false, with nothing launched, when it does not apply.
 static int search_run_bits(blg_ctx *c, blg_search *s, int dtype, void *d_out, bool *done) {
     *done = false;
-    if (!s->tt || !s->bits_mem || bits_table_bytes(s->nsym, s->bits_longest) > kBitsMaxTable) return BLG_OK;
-    if (c->tuning || use_prefix(s) || !bits_faster(c, s)) return BLG_OK;
+    if (use_prefix(s) || !bits_applies(c, s)) return BLG_OK;
     BitSearch B{};
     B.Q = s->q.d;
     B.nq = s->bits_nq;
@@ -1742,9 +1791,8 @@ static int search_run_bits(blg_ctx *c, blg_search *s, int dtype, void *d_out, bo
     void *scratch = nullptr;
     if (s->bits_longest > 64) {
         B.scratch_words = bits_scratch_words(s->max_len);
-        const size_t bytes = sizeof(uint32_t) * (size_t)B.scratch_words * (size_t)bits_warps(c->sms);
-        if (bytes > kBitsMaxScratch) return BLG_OK;
-        CK(dev_alloc(c, &scratch, bytes), "cudaMallocAsync(stripe deltas)");
+        CK(dev_alloc(c, &scratch, sizeof(uint32_t) * (size_t)B.scratch_words * (size_t)bits_warps(c->sms)),
+           "cudaMallocAsync(stripe deltas)");
         B.scratch = (uint32_t *)scratch;
     }
     const cudaError_t e = launch(c, "search_bits", [&] {
@@ -1867,7 +1915,7 @@ static int search_run(blg_ctx *c, blg_search *s, int k, int dtype, void *d_out, 
                }), "search_lanes");
         } else {
             const int qpb = pick_qpb(c, k_.nw, k_.nq, s->nc);
-            if (!hask && use_prefix(s) && search_pfx_supported(k_.nw)) {
+            if (!hask && class_prefix(c, s, k_)) {
                 // exact short queries over the prefix-sorted choices
                 CK(cudaMemsetAsync(s->pfx_work, 0, sizeof(unsigned long long), c->stream), "reset work");
                 CK(launch(c, "search_pfx", [&] {
