@@ -270,6 +270,15 @@ static cudaError_t launch(blg_ctx *c, const char *name, F &&fn) {
     return e;
 }
 
+// One launch under two profile labels: the stage it is, and the kernel that runs it.
+template <typename F>
+static cudaError_t launch_as(blg_ctx *c, const char *stage, const char *name, F &&fn) {
+    return launch(c, stage, [&] {
+        c->launches--;
+        return launch(c, name, fn);
+    });
+}
+
 static cudaError_t dev_alloc(blg_ctx *c, void **p, size_t bytes) {
     if (c->fault_alloc_after >= 0 && c->fault_alloc_after-- == 0) {   // injected failure (tests)
         *p = nullptr;
@@ -791,8 +800,10 @@ static int pairs_run_range(blg_ctx *c, blg_pairs *p, const DevStrings &A, const 
     if (A.n == 0) return BLG_OK;
     const bool use_tile = !exit_log && pairs_use_tile(c, p);
     if (!exit_log && pairs_use_reach(c, p, k, use_tile)) {
-        CK(launch(c, "pairs_solve", [&] { return launch_pairs_reach(c->stream, c->sms, A, B, (double)p->len_max_side / (double)p->n, k, dtype, d_out, c->d_status); }),
-           "pairs_solve");
+        CK(launch_as(c, "pairs_solve", "pairs_reach", [&] {
+               return launch_pairs_reach(c->stream, c->sms, A, B, (double)p->len_max_side / (double)p->n, k, dtype, d_out,
+                                         c->d_status);
+           }), "pairs_reach");
         return BLG_OK;
     }
     if (k < 0 && !exit_log && !use_tile && pairs_use_bands(c, p)) return pairs_run_bands(c, p, A, B, dtype, d_out);

@@ -1,0 +1,38 @@
+"""Which kernel a pairs run takes by its size, lengths and max_dist (blg_api.cu:
+pairs_use_reach), on both sides of each limit, by the profile's labels. Results
+are compared for equality on every route."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import oracle
+from editdist_bench_gb300 import _lib, workloads as W
+from test_gpu_prefix import _labels
+from test_search_filter import TEXT
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(gpu, a, b, k, dtype="uint8"):
+    s = gpu.PairsBatch(a, b)
+    out = s.alloc(dtype)
+    labels = _labels(_lib.context(), lambda: s.run(out, max_dist=k))
+    np.testing.assert_array_equal(out.get(), oracle.saturate(oracle.pairs(a, b, k, threads=8), dtype))
+    return labels
+
+
+def _near(rng, n, lo, hi, alphabet, rate=0.05):
+    a = W.random_strings(rng, rng.integers(lo, hi + 1, n), alphabet)
+    return a, W.mutate(rng, a, rate, alphabet)
+
+
+# words (the tile kernel from k = 3), near-copies of longer strings, many and few
+@pytest.mark.parametrize("n,lo,hi,ks", [(5000, 4, 20, {2: True, 3: False}), (40000, 40, 60, {8: True, 10: False}),
+                                        (1 << 15, 40, 60, {12: True, 17: False})])
+def test_reach_limits(gpu, n, lo, hi, ks):
+    a, b = _near(np.random.default_rng(n), n, lo, hi, W.DNA)
+    for k, reach in ks.items():
+        labels = _run(gpu, a, b, k)
+        assert ("pairs_reach" in labels) == reach, (k, labels)
+        assert not reach or "pairs_solve" in labels, labels       # the stage it is, beside the kernel
