@@ -128,6 +128,8 @@ constexpr size_t kBitsMaxScratch = size_t(512) << 20;
 // 65536: 498 against 183): tests/test_gpu_prefix.py expects this kernel there.
 constexpr double kBitsPfxSaving = 0.45;
 constexpr int kPfxMinQueries = 33, kPfxMaxQueries = 64;
+// Exact pairs in bands first from so many pairs on (pairs_use_bands).
+constexpr int64_t kBandsMinPairs = 1 << 16;
 // Tensor-core filter: pairs below which its launch costs more than it saves.
 constexpr double kFltMinPairs = 1e6;
 // Thresholded searches of at most this many pairs run in one launch
@@ -163,8 +165,7 @@ struct blg_pairs {
     // known; the banded solver's one-row-per-byte variant needs at most 15)
     uint32_t *d_alpha = nullptr;
     int nsym = -1;
-    // resident sets: a sample's pairs share 4-grams (pairs_related)
-    bool related = false;
+    int unrelated = 0;            // of a sample (pairs_sample)
     // resident runs as a CUDA graph (pairs_run_graph): the launches of one
     // run, captured once its parameters repeat, replayed while they stay
     struct GraphKey {
@@ -550,11 +551,50 @@ static int pairs_classify(blg_ctx *c, const int64_t *oa, const int64_t *ob, int6
     return BLG_OK;
 }
 
+// A sample of a set's pairs: how many look unrelated, by the distance of their
+// first 64 bytes (one word of Myers' recurrence) against 45% of them (unrelated DNA:
+// 53%, text: 90%; edits at a rate of 0.3: 25%). Decides routes, never a result.
+constexpr int kPairSamples = 64;
+
+static bool prefix_unrelated(const uint8_t *a, int64_t la, const uint8_t *b, int64_t lb) {
+    const int m = (int)std::min<int64_t>(64, la), n = (int)std::min<int64_t>(64, lb);
+    if (m == 0 || n == 0 || (m == n && memcmp(a, b, (size_t)m) == 0)) return false;
+    uint64_t peq[256] = {}, pv = ~0ull, mv = 0;
+    for (int i = 0; i < m; i++) peq[a[i]] |= 1ull << i;
+    int d = m;
+    for (int j = 0; j < n; j++) {
+        const uint64_t eq = peq[b[j]], xv = eq | mv, xh = (((eq & pv) + pv) ^ pv) | eq;
+        uint64_t ph = mv | ~(xh | pv), mh = pv & xh;
+        d += (int)(ph >> (m - 1) & 1) - (int)(mh >> (m - 1) & 1);
+        ph = ph << 1 | 1;
+        mh <<= 1;
+        pv = mh | ~(xv | ph);
+        mv = ph & xv;
+    }
+    return 20 * d > 9 * std::max(m, n);
+}
+
+// k: of the one call (a resident set's runs may have any: kAnyDist). The strings are
+// read only where a rule asks (pairs_use_bands).
+constexpr int kAnyDist = -2;
+static void pairs_sample(const uint8_t *ba, const int64_t *oa, const uint8_t *bb, const int64_t *ob, int k, blg_pairs *p) {
+    if (!p->trusted || p->too_long || p->n == 0) return;
+    const bool bands = k == kAnyDist && p->cap[0] > 0 && (p->n >= kBandsMinPairs || p->cap[1] == 0);
+    if (!bands) return;
+    for (int x = 0; x < kPairSamples; x++) {
+        const int64_t i = p->n * x / kPairSamples;
+        const int64_t la = oa[i + 1] - oa[i], lb = ob[i + 1] - ob[i];
+        const bool equal = la == lb && (la == 0 || memcmp(ba + oa[i], bb + ob[i], (size_t)la) == 0);
+        p->unrelated += !equal && prefix_unrelated(ba + oa[i], la, bb + ob[i], lb);
+    }
+}
+
 static int pairs_upload(blg_ctx *c, const uint8_t *ba, const int64_t *oa, const uint8_t *bb,
                         const int64_t *ob, int64_t n, blg_pairs *p) {
     int rc = upload_strings(c, ba, oa, n, p->a);
     if (!rc) rc = upload_strings(c, bb, ob, n, p->b);
     if (!rc) rc = pairs_classify(c, oa, ob, n, p);
+    if (!rc) pairs_sample(ba, oa, bb, ob, kAnyDist, p);
     return rc;
 }
 
@@ -676,45 +716,27 @@ static bool pairs_use_tile(const blg_ctx *c, const blg_pairs *p) {
     return c->sched == BLG_SCHED_AUTO && 4 * p->short_pairs >= 3 * p->n;
 }
 
-// Whether the pairs of a set are mostly near each other, from 32 of them: their
-// sets of 6-grams (4096 hashed bins) differ in well under what unrelated
-// strings' would; edits at a rate r keep (1 - r)^6 of the grams. Decides a
-// route, never a result.
-static bool pairs_related(const uint8_t *ba, const int64_t *oa, const uint8_t *bb, const int64_t *ob, int64_t n) {
-    constexpr int kGram = 6, kBins = 4096;
-    const int64_t samples = std::min<int64_t>(32, n);
-    double differ = 0.0, expected = 0.0;
-    for (int64_t x = 0; x < samples; x++) {
-        const int64_t i = n * x / samples;
-        uint64_t set[2][kBins / 64] = {};
-        int bits[2] = {0, 0}, diff = 0;
-        for (int t = 0; t < 2; t++) {
-            const uint8_t *p = (t ? bb : ba) + (t ? ob : oa)[i];
-            const int64_t len = std::min<int64_t>(512, (t ? ob : oa)[i + 1] - (t ? ob : oa)[i]);
-            for (int64_t y = 0; y + kGram <= len; y++) {
-                uint32_t h = 0;
-                for (int z = 0; z < kGram; z++) h = (h ^ p[y + z]) * 0x9E3779B1u;
-                set[t][h >> 26] |= 1ull << (h >> 20 & 63u);
-            }
-            for (uint64_t w : set[t]) bits[t] += __builtin_popcountll(w);
-        }
-        for (int w = 0; w < kBins / 64; w++) diff += __builtin_popcountll(set[0][w] ^ set[1][w]);
-        differ += diff;
-        expected += bits[0] + bits[1] - 2.0 * bits[0] * bits[1] / kBins;
-    }
-    return expected > 0.0 && differ < 0.8 * expected;
-}
-
 // Bands first, for exact runs of a resident set (its alphabet and a sample are
 // known) of near pairs with patterns past one word. Bands / full width,
 // microseconds: 250007 pairs of 8 to 256 bytes with up to 30% edits 243 / 355,
 // 10^6 829 / 1197, 250000 of 60 to 120 with up to 10% 81 / 128. Few pairs wait for the
 // longer chain of kernels (20000 of 8 to 256 147 / 120, 100000 172 / 180) unless no
 // pattern is longer than 128 (20000 of 4 to 80 44 / 62); unrelated pairs leave both
-// bands late (60 to 250 bytes: 643 / 470).
+// bands late (60 to 250 bytes: 643 / 470), and a few of them make every kernel of the
+// chain run. With one pair in ten unrelated, DNA, then text: 250000 of 8 to 256 253 /
+// 352, 316 / 360; 70000 182 / 139, 193 / 140; 250000 of 4 to 80 77 / 88, 124 / 90; 70000
+// of 60 to 120 89 / 87, 100 / 89, of 200 to 400 269 / 434, 266 / 437; 20000 of 60 to 120
+// 102 / 66. What the sample may hold follows from these. A few that it does not show
+// cost as much: one in 100 of 20000 of 60 to 120 100 / 66, of 250000 texts of 4 to 80
+// 122 / 89.
 static bool pairs_use_bands(const blg_ctx *c, const blg_pairs *p) {
-    return c->sched == BLG_SCHED_AUTO && !c->tuning && p->trusted && !p->too_long && p->cap[0] > 0 && p->nsym >= 0 &&
-           p->related && (p->n >= (1 << 16) || p->cap[1] == 0);
+    if (c->sched != BLG_SCHED_AUTO || c->tuning || !p->trusted || p->too_long || p->cap[0] == 0 || p->nsym < 0) return false;
+    if (p->n < kBandsMinPairs) return p->cap[1] == 0 && p->unrelated <= kPairSamples / 32;
+    const int64_t mean = p->len_max_side / p->n;
+    int room = kPairSamples / 4;
+    if (p->nsym > kBandSymbols) room = mean < 128 ? 0 : mean >= 200 ? room : p->n >= 200000 ? kPairSamples / 8 : 3;
+    else if (mean >= 128 && mean < 200 && p->n < (1 << 17)) room = 1;
+    return p->unrelated <= room;
 }
 
 // Exact runs with long patterns under the automatic schedule: bands first
@@ -864,6 +886,7 @@ static int pairwise_pipelined(blg_ctx *c, const uint8_t *ba, const int64_t *oa, 
         if (!rc && cudaEventRecord(ev[1 + ch], c->up) != cudaSuccess) rc = fail(c, BLG_ERR_CUDA, "event");
     }
     if (!rc) rc = pairs_classify(c, oa, ob, n, p);          // overlaps the copies
+    if (!rc) pairs_sample(ba, oa, bb, ob, std::max(k, -1), p);
     for (int ch = 0; ch <= nch && !rc; ch++) {
         if (ch < nch) {
             const int64_t i0 = n * ch / nch, i1 = n * (ch + 1) / nch;
@@ -3116,7 +3139,6 @@ int blg_pairs_upload(blg_ctx *c, const uint8_t *ba, const int64_t *oa, const uin
     // synchronises): the device copy is the data the host pass checked,
     // whatever the caller does with its buffers.
     if (!rc) rc = pairs_learn_alphabet(c, p);
-    if (!rc && n > 0 && p->trusted) p->related = pairs_related(ba, oa, bb, ob, n);
     if (!rc && cudaStreamSynchronize(c->stream) != cudaSuccess) rc = fail(c, BLG_ERR_CUDA, "upload");
     if (rc) {
         pairs_release(c, p);
@@ -3385,6 +3407,7 @@ int blg_pairwise(blg_ctx *c, const uint8_t *ba, const int64_t *oa, const uint8_t
         if (!rc) rc = pairwise_pipelined(c, ba, oa, bb, ob, n, max_dist, dtype, out_host, d_out, &p);
     } else {
         if (!rc) rc = pairs_classify(c, oa, ob, n, &p);
+        if (!rc) pairs_sample(ba, oa, bb, ob, std::max(max_dist, -1), &p);
         if (!rc) rc = upload_strings(c, ba, oa, n, p.a);
         if (!rc) rc = upload_strings(c, bb, ob, n, p.b);
         if (!rc) rc = pairs_run(c, &p, max_dist, u4 ? BLG_UINT8 : dtype, u4 ? d8 : d_out);

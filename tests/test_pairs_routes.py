@@ -28,7 +28,7 @@ def _near(rng, n, lo, hi, alphabet, rate=0.05):
 
 
 # words (the tile kernel from k = 3), near-copies of longer strings, many and few
-@pytest.mark.parametrize("n,lo,hi,ks", [(5000, 4, 20, {2: True, 3: False}), (40000, 40, 60, {8: True, 10: False}),
+@pytest.mark.parametrize("n,lo,hi,ks", [(5000, 4, 20, {2: True, 3: False}), (40000, 40, 60, {9: True, 10: False}),
                                         (1 << 15, 40, 60, {12: True, 17: False})])
 def test_reach_limits(gpu, n, lo, hi, ks):
     a, b = _near(np.random.default_rng(n), n, lo, hi, W.DNA)
@@ -36,3 +36,17 @@ def test_reach_limits(gpu, n, lo, hi, ks):
         labels = _run(gpu, a, b, k)
         assert ("pairs_reach" in labels) == reach, (k, labels)
         assert not reach or "pairs_solve" in labels, labels       # the stage it is, beside the kernel
+
+
+# many pairs of another origin, or at most one in 50
+@pytest.mark.parametrize("n,share,alphabet,bands", [(20000, 0.25, W.DNA, False), (20000, 0.0, W.DNA, True), (70000, 0.5, W.DNA, False),
+                                                    (70000, 0.02, W.DNA, True), (70000, 0.1, TEXT, False), (70000, 0.0, TEXT, True)])
+def test_bands_leave_mixed_sets(gpu, n, share, alphabet, bands):
+    rng = np.random.default_rng(7)
+    a, b = _near(rng, n, 60, 90, alphabet)
+    other = np.flatnonzero(rng.random(n) < share)
+    order = np.arange(n)
+    order[other] += n
+    b = W.take(W.concat(b, W.random_strings(rng, np.diff(a[1]), alphabet)), order)
+    labels = _run(gpu, a, b, None, "int32")
+    assert ("pairs_bands" in labels) == bands, labels
