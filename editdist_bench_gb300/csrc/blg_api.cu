@@ -128,8 +128,9 @@ constexpr size_t kBitsMaxScratch = size_t(512) << 20;
 // 65536: 498 against 183): tests/test_gpu_prefix.py expects this kernel there.
 constexpr double kBitsPfxSaving = 0.45;
 constexpr int kPfxMinQueries = 33, kPfxMaxQueries = 64;
-// Exact pairs in bands first from so many pairs on (pairs_use_bands).
-constexpr int64_t kBandsMinPairs = 1 << 16;
+// Exact pairs in bands first from so many pairs on; furthest-reaching points with
+// the larger thresholds up to so many (pairs_use_bands, pairs_use_reach).
+constexpr int64_t kBandsMinPairs = 1 << 16, kReachFewPairs = 1 << 15;
 // Tensor-core filter: pairs below which its launch costs more than it saves.
 constexpr double kFltMinPairs = 1e6;
 // Thresholded searches of at most this many pairs run in one launch
@@ -166,6 +167,8 @@ struct blg_pairs {
     uint32_t *d_alpha = nullptr;
     int nsym = -1;
     int unrelated = 0;            // of a sample (pairs_sample)
+    int equal = 0;
+    int stride = 0;               // 32, 128: most of a side's strings have one length, a multiple of that many bytes
     // resident runs as a CUDA graph (pairs_run_graph): the launches of one
     // run, captured once its parameters repeat, replayed while they stay
     struct GraphKey {
@@ -574,17 +577,33 @@ static bool prefix_unrelated(const uint8_t *a, int64_t la, const uint8_t *b, int
     return 20 * d > 9 * std::max(m, n);
 }
 
+// Whether most of a side's strings have one length that is a multiple of 128, or of
+// 32 (0: no).
+static int common_stride(const int64_t *off, int64_t n) {
+    const int64_t len = off[n / 2 + 1] - off[n / 2];
+    if (len <= 0 || len % 32) return 0;
+    int same = 0;
+    for (int x = 0; x < kPairSamples; x++) {
+        const int64_t i = n * x / kPairSamples;
+        same += off[i + 1] - off[i] == len;
+    }
+    return 4 * same < 3 * kPairSamples ? 0 : len % 128 ? 32 : 128;
+}
+
 // k: of the one call (a resident set's runs may have any: kAnyDist). The strings are
-// read only where a rule asks (pairs_use_bands).
+// read only where a rule asks (pairs_use_bands, pairs_use_reach).
 constexpr int kAnyDist = -2;
 static void pairs_sample(const uint8_t *ba, const int64_t *oa, const uint8_t *bb, const int64_t *ob, int k, blg_pairs *p) {
     if (!p->trusted || p->too_long || p->n == 0) return;
+    p->stride = std::max(common_stride(oa, p->n), common_stride(ob, p->n));
     const bool bands = k == kAnyDist && p->cap[0] > 0 && (p->n >= kBandsMinPairs || p->cap[1] == 0);
-    if (!bands) return;
+    const bool reach = p->stride && p->n > kReachFewPairs && (k == kAnyDist || (k >= 0 && k <= 9));
+    if (!(bands || reach)) return;
     for (int x = 0; x < kPairSamples; x++) {
         const int64_t i = p->n * x / kPairSamples;
         const int64_t la = oa[i + 1] - oa[i], lb = ob[i + 1] - ob[i];
         const bool equal = la == lb && (la == 0 || memcmp(ba + oa[i], bb + ob[i], (size_t)la) == 0);
+        p->equal += equal;
         p->unrelated += !equal && prefix_unrelated(ba + oa[i], la, bb + ob[i], lb);
     }
 }
@@ -763,15 +782,28 @@ static int pairs_run_bands(blg_ctx *c, blg_pairs *p, const DevStrings &A, const 
 // Furthest-reaching points (k_pairs_reach) under the automatic schedule while k
 // is small: its steps grow with k^2, the banded loop's columns hardly. One
 // kernel / prep, order and banded loop, microseconds: 2^20 pairs of 8 to 256
-// bytes 102 / 244 at k = 2, 159 / 307 at 4, 302 / 385 at 8, 383 / 407 at 10, 474
-// / 436 at 12; 300000 lines of 40 to 100 25 / 79, 41 / 84, 72 / 86, 89 / 87; few
-// pairs, where three launches wait for one another, 20000 of 8 to 256 49 / 121
-// at 12. Against the short-pair tile kernel (2^20 words of 10 to 30) 35 / 48
-// at 2, 46 / 49 at 3, 62 / 50 at 4. Pairs that a kernel would refuse by
-// their trimmed length (shorter string above 2048) take the other paths.
+// bytes 102 / 244 at k = 2, 159 / 307 at 4, 302 / 385 at 8, 383 / 407 at 10; few
+// pairs, where three launches wait for one another, 20000 of 8 to 256 49 / 121 at 12,
+// 1000 of 40 to 100 27 / 52 at 16. Unrelated pairs of like length walk every number of
+// edits up to k, where the banded loop leaves after some 2 k columns. That matters
+// where the lanes' strings lie a
+// multiple of 32 bytes apart and share a few banks: 10^6 unrelated texts of 64 150 /
+// 177 at k = 4, 203 / 178 at 5, 448 / 177 at 8, half of them unrelated 289 / 224 (of 40
+// to 100, 200000 31 / 65); 20000 39 / 38 at 12, 50 / 38 at 14; multiples of 128 share
+// them all: 10^6 of 128 279 / 248 at 4, 331 / 267 if equal, 20000 of 256 70 / 41 at
+// 12. 10^6 texts of 20 to 60 176 / 168 at k = 9, 200000 of 40 to 100 37 / 64. Strings
+// whose groups of 32 do not fit the stage are read in place, a sector a step: 200000
+// equal pairs of 500 to 600 508 / 235, but few pairs with k up to 9 gain (20000 of 600
+// to 1200, k = 8: 24 to 93 / 40 to 171). Against the short-pair tile kernel (2^20 words of 10 to 30) 35 /
+// 48 at 2, 46 / 49 at 3, 62 / 50 at 4. Pairs that a kernel would refuse by their
+// trimmed length (shorter string above 2048) take the other paths.
 static bool pairs_use_reach(const blg_ctx *c, const blg_pairs *p, int k, bool tile) {
     if (k < 0 || c->sched != BLG_SCHED_AUTO || c->tuning || !p->trusted || p->too_long) return false;
-    return k <= (tile ? 2 : p->n <= (1 << 15) ? 16 : 9);
+    if (tile) return k <= 2;
+    if (32 * p->len_max_side > kReachMaxSpan * p->n) return p->n <= kReachFewPairs && k <= 9;
+    if (p->n <= kReachFewPairs) return k <= (p->stride == 128 ? 8 : p->stride == 32 ? 12 : 16);
+    if (p->stride && 16 * p->unrelated > 3 * kPairSamples) return k <= (p->stride == 128 ? 3 : 4);
+    return k <= (p->n <= (1 << 18) ? 9 : 8) && !(p->stride == 128 && 2 * p->equal > kPairSamples);
 }
 
 // One launch of the direct pairs path (tile or staged kernel + the long-pair

@@ -112,6 +112,10 @@ struct SearchClass {
 // bytes outside the set); larger alphabets use nibble rows.
 constexpr int kBandSymbols = 15;
 
+// Bytes of each side that k_pairs_reach stages for a warp's 32 pairs; longer
+// groups are read in place.
+constexpr int kReachMaxSpan = 12288;
+
 // Query word classes of the sequential search kernels (patterns of 1..8
 // 64-bit words); longer queries run lane-spread. A thresholded run plans and
 // solves the survivors of all its sequential classes in one launch each.

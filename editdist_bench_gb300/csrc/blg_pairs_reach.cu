@@ -24,7 +24,6 @@
 namespace blg {
 
 constexpr int kReachThreads = 128;
-constexpr int kReachMaxSpan = 12288;             // staged bytes per side and warp; longer groups are read in place
 
 __global__ void __launch_bounds__(kReachThreads)
     k_pairs_reach(DevStrings A, DevStrings B, int span, int k, int dtype, void *out, uint32_t *status) {

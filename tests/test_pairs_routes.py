@@ -38,6 +38,28 @@ def test_reach_limits(gpu, n, lo, hi, ks):
         assert not reach or "pairs_solve" in labels, labels       # the stage it is, beside the kernel
 
 
+# what a sample finds unrelated among strings 64 bytes apart, strings too long for the
+# stage, both sides of each limit
+@pytest.mark.parametrize("n,lo,hi,related,ks", [(40000, 64, 64, False, {4: True, 5: False, 9: False}),
+                                                (40000, 64, 64, True, {9: True, 10: False}),
+                                                (40000, 128, 128, False, {3: True, 4: False}),
+                                                (2000, 128, 128, False, {8: True, 9: False}),
+                                                (2000, 64, 64, False, {12: True, 13: False}),
+                                                (40000, 64, 72, False, {9: True, 10: False}),
+                                                (2000, 63, 63, False, {16: True, 17: False}),
+                                                (40000, 400, 420, True, {3: False}),
+                                                (1000, 400, 420, True, {9: True, 10: False})])
+def test_reach_leaves_what_it_would_slow_down(gpu, n, lo, hi, related, ks):
+    rng = np.random.default_rng(n + lo)
+    a, b = _near(rng, n, lo, hi, TEXT, 0.01)
+    if not related:
+        b = W.random_strings(rng, np.diff(a[1]), TEXT)
+    for k, reach in ks.items():
+        labels = _run(gpu, a, b, k)
+        assert ("pairs_reach" in labels) == reach, (k, labels)
+        np.testing.assert_array_equal(gpu.pairwise_packed(a, b, max_dist=k), oracle.pairs(a, b, k, threads=8))
+
+
 # many pairs of another origin, or at most one in 50
 @pytest.mark.parametrize("n,share,alphabet,bands", [(20000, 0.25, W.DNA, False), (20000, 0.0, W.DNA, True), (70000, 0.5, W.DNA, False),
                                                     (70000, 0.02, W.DNA, True), (70000, 0.1, TEXT, False), (70000, 0.0, TEXT, True)])
@@ -50,3 +72,8 @@ def test_bands_leave_mixed_sets(gpu, n, share, alphabet, bands):
     b = W.take(W.concat(b, W.random_strings(rng, np.diff(a[1]), alphabet)), order)
     labels = _run(gpu, a, b, None, "int32")
     assert ("pairs_bands" in labels) == bands, labels
+
+
+def test_reach_leaves_copies_that_share_all_banks(gpu):
+    a = W.random_strings(np.random.default_rng(3), np.full(40000, 128))
+    assert "pairs_reach" not in _run(gpu, a, a, 2)
