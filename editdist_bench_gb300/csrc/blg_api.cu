@@ -133,11 +133,6 @@ constexpr int kPfxMinQueries = 33, kPfxMaxQueries = 64;
 constexpr int64_t kBandsMinPairs = 1 << 16, kReachFewPairs = 1 << 15;
 // Tensor-core filter: pairs below which its launch costs more than it saves.
 constexpr double kFltMinPairs = 1e6;
-// Thresholded searches of at most this many pairs run in one launch
-// (k_search_small). One launch / the survivor kernel, microseconds: 1 x 20000
-// words at k = 2 5 / 77, 64 x 20000 DNA of 30 to 120 at k = 2 22 / 42, 30 x 200000
-// (6 M pairs) 50 / 42, words 46 / 58.
-constexpr double kSmallPairs = 4e6;
 
 struct OwnedStrings {
     DevStrings d;
@@ -1622,30 +1617,53 @@ static int pick_qpb(blg_ctx *c, int nw, int nq_cls, int64_t nc) {
     return (int)qpb;
 }
 
-// Launch the current classes' kernels; the max_dist fill covers rows [q0, q1)
-// (all rows by default: the classes hold every query).
-// Survivors per job of the thresholded search: the tuned size, halved
-// (down to 128, a warp's scan step) while the run would have fewer than 4 jobs
-// per warp of the persistent grid, so small searches still spread over the GPU
-// (64 x 200000 lines of 3 to 40 bytes at k = 3: 68 us, 115 with jobs of 1024 at
-// the least; 1000 x 100000: 303 and 309). The
-// survivor count comes from the host copies of the length histogram.
-static int survivor_job_size(blg_ctx *c, const blg_search *s, int k) {
-    int64_t total = 0;
+// The pairs of the sequential queries and the choices within k of their length (from
+// the host copy of the length histogram), and the columns of their query's length.
+struct Window {
+    int64_t pairs = 0;
+    double columns = 0.0;
+};
+
+static Window window_of(const blg_search *s, int k) {
+    Window w;
     const int64_t nl = s->n_len;
     for (auto &k_ : s->cls) {
         if (k_.lanes) continue;
         for (int32_t m : k_.h_qlen) {
-            int64_t a = m - k - s->min_len, b = m + k - s->min_len + 1;
-            a = std::max<int64_t>(0, std::min(a, nl));
-            b = std::max<int64_t>(0, std::min(b, nl));
-            if (b > a) total += s->h_lstart[b] - s->h_lstart[a];
+            const int64_t a = std::max<int64_t>(0, std::min(m - k - s->min_len, nl));
+            const int64_t b = std::max<int64_t>(a, std::min(m + k - s->min_len + 1, nl));
+            const int64_t n = s->h_lstart[b] - s->h_lstart[a];
+            w.pairs += n;
+            w.columns += (double)n * (double)m;
         }
     }
+    return w;
+}
+
+// Survivors per job of the thresholded search: the tuned size, halved
+// (down to 128, a warp's scan step) while the run would have fewer than 4 jobs
+// per warp of the persistent grid, so small searches still spread over the GPU
+// (64 x 200000 lines of 3 to 40 bytes at k = 3: 68 us, 115 with jobs of 1024 at
+// the least; 1000 x 100000: 303 and 309).
+static int survivor_job_size(blg_ctx *c, const Window &w, int k) {
     const int64_t warps = (int64_t)c->sms * surv_ctas(c, k) * 8;
     int job = c->tune.lpt_job;
-    while (job > 128 && total < 4 * warps * (int64_t)job) job >>= 1;
+    while (job > 128 && w.pairs < 4 * warps * (int64_t)job) job >>= 1;
     return job;
+}
+
+// Whether a thresholded search of `pairs` pairs runs in one launch (k_search_small).
+// One launch / the survivor kernel, microseconds: 1 x 20000 words at k = 2 5 / 77, 64 x
+// 20000 DNA of 30 to 120 22 / 42. It has a thread per pair, so the pairs outside
+// the length window cost it as much as the others' test (64 x 40000 of 300 to 512
+// at k = 3: 62 / 51, of 3 to 16 29 / 102), and a warp walks the columns of whichever of
+// its lanes passed the test, where the survivor kernel packs those. Every length
+// equal and a sixteenth of the pairs related (reads of 64 of 16 families), 64 x 40000, 64
+// x 20000: k = 1 19 / 38, 15 / 34; k = 2 53 / 47, 34 / 41; k = 3 107 / 54, 60 / 46 (16 x
+// 60000: 54 / 45), texts at k = 8 104 / 85, at 12 114 / 120 (64 x 40000 218 / 204).
+static bool search_small(const blg_search *s, const Window &w, double pairs, int k) {
+    const bool short_choices = s->min_len + s->n_len - 1 <= 64;
+    return pairs <= (short_choices ? 4e6 : 1.7e6) && w.columns <= (k <= 1 ? 2.4e8 : k == 2 ? 7e7 : k < 12 ? 4e7 : 1.1e8);
 }
 
 // The sequential (not lane-spread) query classes of a search, for the
@@ -1870,6 +1888,8 @@ static int search_run_bits(blg_ctx *c, blg_search *s, int dtype, void *d_out, bo
     return BLG_OK;
 }
 
+// Launch the current classes' kernels; the max_dist fill covers rows [q0, q1)
+// (all rows by default: the classes hold every query).
 static int search_run(blg_ctx *c, blg_search *s, int k, int dtype, void *d_out, int64_t q0, int64_t q1) {
     if (!dtype_ok(dtype)) return fail(c, BLG_ERR_ARG, "dtype must be int32, uint16 or uint8");
     if (s->nq == 0 || s->nc == 0) return BLG_OK;
@@ -1896,13 +1916,14 @@ static int search_run(blg_ctx *c, blg_search *s, int k, int dtype, void *d_out, 
         const bool band = k <= 31 && C.n > 0;
         int64_t seq_q = 0;
         for (int i = 0; i < C.n; i++) seq_q += C.cls[i].nq;
-        const bool small = band && !c->tuning && (double)seq_q * (double)s->nc <= kSmallPairs && seq_q <= 65535;
+        const Window win = band ? window_of(s, k) : Window{};
+        const bool small = band && !c->tuning && seq_q <= 65535 && search_small(s, win, (double)seq_q * (double)s->nc, k);
         if (small)
             CK(launch(c, "search_small", [&] {
                    return launch_search_small(c->stream, C, s->cs.d, s->perm, s->ccnt, s->qcnt, k, dtype, d_out, s->nc,
                                               c->d_status);
                }), "search_small");
-        const int job = band && !small ? survivor_job_size(c, s, k) : 1024;
+        const int job = band && !small ? survivor_job_size(c, win, k) : 1024;
         const FilterPlan fp = band && !small ? filter_plan(c, s, C, k) : FilterPlan{};
         const bool filter = fp.pays;
         if (filter) {
@@ -2110,7 +2131,7 @@ static int search_matches_list(blg_ctx *c, blg_search *s, int k, blg_match *d_ou
     const SurvClasses C = seq_classes(s);
     if (C.n == 0 || C.n != (int)s->cls.size()) return BLG_OK;    // a lane-spread class: the dense path
     if (class_queries(s) != s->nq) return BLG_OK;                  // not every query's class: the dense path
-    const int job = survivor_job_size(c, s, k);
+    const int job = survivor_job_size(c, window_of(s, k), k);
     const ResultList L{c->rl_hdr + 2, c->rl_hdr, c->rl_cap};
     CK(cudaMemsetAsync(c->rl_hdr, 0, 2 * sizeof(unsigned long long), c->stream), "clear list");
     unsigned long long cnt = 0;
@@ -3340,7 +3361,7 @@ int blg_sched_train_search(blg_ctx *c, blg_search *s, int32_t max_dist, int32_t 
     CK(cudaMemsetAsync(nrows, 0, sizeof(int64_t), c->stream), "memset");
     SurvRows R{(half *)x, (float *)y, max_rows, (int64_t *)nrows,
                (int)std::min<int64_t>(INT32_MAX, std::max<int64_t>(1, (survivors + max_rows - 1) / max_rows))};
-    const int job = survivor_job_size(c, s, max_dist);
+    const int job = survivor_job_size(c, window_of(s, max_dist), max_dist);
     CK(launch(c, "surv_plan", [&] {
            return launch_surv_plan(c->stream, C, s->lstart, s->min_len, s->n_len, max_dist, job);
        }), "surv_plan");

@@ -1,0 +1,31 @@
+"""Which kernel a thresholded search takes by its size, lengths and data
+(blg_api.cu: search_small, filter_plan), by the profile's labels, and the dense
+output and result list of each. Results are compared for equality."""
+import numpy as np
+import pytest
+
+import oracle
+from editdist_bench_gb300 import workloads as W
+from test_search_filter import TEXT, _run, _sets
+
+pytestmark = pytest.mark.gpu
+
+
+def _families(rng, nq, nc, length, families, rate=0.08, alphabet=W.DNA):
+    """Every string a mutant of one of some stems, cut or filled to one length."""
+    stems = W.random_strings(rng, np.full(families, length), alphabet)
+    fix = lambda p: (np.concatenate([np.resize(np.append(p[0][p[1][i]:p[1][i + 1]], alphabet[0]), length)
+                                     for i in range(len(p[1]) - 1)]), np.arange(len(p[1])) * length)
+    return tuple(fix(W.mutate(rng, W.take(stems, rng.integers(0, families, n)), rate, alphabet)) for n in (nq, nc))
+
+
+# one launch or the survivor kernel: pairs in all, columns within the window, k
+@pytest.mark.parametrize("nq,nc,length,ks", [(64, 20000, 64, {1: True, 2: False, 3: False}), (16, 30000, 64, {2: True, 3: True}),
+                                             (64, 40000, 8, {1: True}), (64, 28000, 80, {0: False})])
+def test_small_search_limits(gpu, nq, nc, length, ks):
+    q, c = _families(np.random.default_rng(nq + nc), nq, nc, length, 16)
+    s = gpu.SearchBatch(q, c)
+    for k, small in ks.items():
+        got, labels = _run(gpu, s, s.alloc("uint8"), k)
+        assert ("search_small" in labels) == small, (k, labels)
+        np.testing.assert_array_equal(got, oracle.saturate(oracle.cross(q, c, k, threads=8), "uint8"))
