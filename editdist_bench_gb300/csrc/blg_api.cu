@@ -229,6 +229,7 @@ struct blg_search {
     int64_t max_len = 0;              // longest choice
     double warp_len = 0.0;            // mean of the longest of 32 neighbours
     int gram_sym = 256;              // the queries' bytes, as that many equally frequent ones (filter_plan)
+    float gram_pass[kSigMaxK + 1] = {};   // by k: share of a sample's pairs whose 4-grams allow it (sample_grams)
     // exact runs, bit-sliced over the queries (k_search_bits): the distinct
     // bytes of the queries (nsym 0: not counted, or too many) and, per class set, the
     // sequential queries by length
@@ -1518,6 +1519,47 @@ static int search_upload_queries(blg_ctx *c, const uint8_t *bq, const int64_t *o
     return BLG_OK;
 }
 
+// Of 32 queries x 64 choices spread over the sets, the share whose signatures differ
+// by at most 8 k, for every k of the filter (filter_plan). The first 512 bytes of a
+// string stand for it. Host work beside the choices' upload.
+static void sample_grams(const uint8_t *bq, const int64_t *oq, int64_t nq, const uint8_t *bc, const int64_t *oc, int64_t nc,
+                         blg_search *s) {
+    if (!s->csig || (double)nq * (double)nc < kFltMinPairs) return;
+    struct Sig {
+        uint64_t w[kSigWords / 2] = {};
+    };
+    auto signature = [](const uint8_t *p, int64_t len) {
+        Sig g;
+        uint32_t gram = 0;
+        for (int64_t i = 0; i < std::min<int64_t>(512, len); i++) {
+            gram = gram << 8 | p[i];
+            if (i < 3) continue;
+            const uint32_t bit = sig_bit(gram);
+            g.w[bit >> 6] |= 1ull << (bit & 63);
+        }
+        return g;
+    };
+    const int64_t qn = std::min<int64_t>(32, nq), cn = std::min<int64_t>(64, nc);
+    Sig q[32];
+    for (int64_t x = 0; x < qn; x++) q[x] = signature(bq + oq[nq * x / qn], oq[nq * x / qn + 1] - oq[nq * x / qn]);
+    int count[kSigMaxK + 1] = {};
+    for (int64_t y = 0; y < cn; y++) {
+        const Sig g = signature(bc + oc[nc * y / cn], oc[nc * y / cn + 1] - oc[nc * y / cn]);
+        for (int64_t x = 0; x < qn; x++) {
+            int diff = 0;
+            for (int w = 0; w < kSigWords / 2; w++) diff += __builtin_popcountll(q[x].w[w] ^ g.w[w]);
+            const int k = (diff + 7) / 8;
+            if (k <= kSigMaxK) count[k]++;
+        }
+    }
+    int sum = 0;
+    for (int k = 0; k <= kSigMaxK; k++) {
+        sum += count[k];
+        s->gram_pass[k] = (float)sum / (float)(qn * cn);
+    }
+}
+
+
 // One-call cdist with host results: queries in chunks of rows; the rows of
 // chunk i go back (stream `down`) while chunk i+1 computes.
 // d4 (optional): 4-bit results. The chunks then compute uint8 rows into
@@ -1531,6 +1573,7 @@ static int cdist_pipelined(blg_ctx *c, const uint8_t *bq, const int64_t *oq, int
     int rc = search_upload_queries(c, bq, oq, nq, s, need);
     if (!rc) rc = search_upload_choices(c, bc, oc, nc, s, need);
     if (rc) return rc;
+    sample_grams(bq, oq, nq, bc, oc, nc, s);
     const size_t row = dtype_size(dtype) * (size_t)nc;
     // Query chunks of relative sizes 4,4,4,4,4,4,4,2,1,1: the last chunk's
     // copy back is the part of the result stream no kernel hides, so the
@@ -1599,6 +1642,7 @@ static int search_upload(blg_ctx *c, const uint8_t *bq, const int64_t *oq, int64
     int rc = search_upload_queries(c, bq, oq, nq, s, need);
     if (!rc && need == NEED_ALL && nq > 0) s->h_oq.assign(oq, oq + nq + 1);   // a resident search keeps them
     if (!rc) rc = search_upload_choices(c, bc, oc, nc, s, need, perm_stage);
+    if (!rc) sample_grams(bq, oq, nq, bc, oc, nc, s);
     if (!rc) rc = search_build_classes(c, oq, 0, nq, s);
     return rc;
 }
@@ -1629,10 +1673,12 @@ static Window window_of(const blg_search *s, int k) {
     const int64_t nl = s->n_len;
     for (auto &k_ : s->cls) {
         if (k_.lanes) continue;
-        for (int32_t m : k_.h_qlen) {
+        for (size_t q = 0, e; q < k_.h_qlen.size(); q = e) {   // queries of one length share a window
+            const int32_t m = k_.h_qlen[q];
+            for (e = q + 1; e < k_.h_qlen.size() && k_.h_qlen[e] == m;) e++;
             const int64_t a = std::max<int64_t>(0, std::min(m - k - s->min_len, nl));
             const int64_t b = std::max<int64_t>(a, std::min(m + k - s->min_len + 1, nl));
-            const int64_t n = s->h_lstart[b] - s->h_lstart[a];
+            const int64_t n = (int64_t)(e - q) * (s->h_lstart[b] - s->h_lstart[a]);
             w.pairs += n;
             w.columns += (double)n * (double)m;
         }
@@ -1784,7 +1830,16 @@ static bool bits_applies(blg_ctx *c, const blg_search *s) {
 // ten: 119 us, 91 per pair). Half the bins where that lets no more through: half
 // the product and half the rows to write, which the warps that read the
 // sums hide; 13 thousand more passers cost far more (1024 x 2^18 reads of 64 at
-// max_dist 4: 246 us folded, 90 whole).
+// max_dist 4: 246 us folded, 90 whole). Related strings pass whatever two unrelated
+// ones do: a sample (sample_grams) says how many, and from one in sixteen of the pairs
+// within the window on (a quarter for strings of up to 72 on average, soon solved), the
+// solver costs more than the per-pair filter, and a list that runs full has gained
+// nothing: three quarters of it, or, where the per-pair filter takes so long that the
+// filter's time hardly shows, all of it and the sample's error (256 x 65536 texts of 150 to 256, k = 12, four
+// families 2241 / 777 us, sixteen 812 / 436; 1024 x 65536 reads of 100 to 140, four
+// families, k = 2 160 / 111; of 64, sixteen families, k = 4 366 / 1221). Where nearly
+// every pair passes it is ahead all the same (2200 x 2205 equal reads of 64, k = 2:
+// 554 / 1267).
 struct FilterPlan {
     bool pays = false, folded = false;
     int nq = 0;
@@ -1852,7 +1907,11 @@ static FilterPlan filter_plan(const blg_ctx *c, const blg_search *s, const SurvC
     f.nq = (int)nq;
     f.folded = pass_folded <= pass + 1e-7 * pairs;
     f.filter_us = 6.0 + std::ceil(tiles / c->sms) * (f.folded ? 0.75 : 1.15);
-    f.pays = pairs >= 1800.0 * tiles && pairs >= kFltMinPairs && pass <= std::min((double)c->pl_cap / 8.0, pairs / 32.0);
+    const double share = s->gram_pass[k], related = share * (double)nq * (double)s->nc;
+    const bool brief = s->c.d.bytes <= 72 * s->nc;
+    const double room = std::min(pairs / (brief ? 4.0 : 16.0), (brief ? 1.25 : 0.75) * (double)c->pl_cap);
+    f.pays = pairs >= 1800.0 * tiles && pairs >= kFltMinPairs && pass <= std::min((double)c->pl_cap / 8.0, pairs / 32.0) &&
+             (related <= room || share >= 0.9);
     return f;
 }
 
@@ -3600,6 +3659,7 @@ int blg_cdist_matches(blg_ctx *c, const uint8_t *bq, const int64_t *oq, int64_t 
     const unsigned need = surv ? NEED_SORTED : NEED_TT;
     int rc = search_upload_queries(c, bq, oq, nq, &s, need);
     if (!rc) rc = search_upload_choices(c, bc, oc, nc, &s, need);
+    if (!rc) sample_grams(bq, oq, nq, bc, oc, nc, &s);
     // the survivor kernel's result list, where the run qualifies
     int64_t total = 0;
     bool listed = false;

@@ -29,3 +29,20 @@ def test_small_search_limits(gpu, nq, nc, length, ks):
         got, labels = _run(gpu, s, s.alloc("uint8"), k)
         assert ("search_small" in labels) == small, (k, labels)
         np.testing.assert_array_equal(got, oracle.saturate(oracle.cross(q, c, k, threads=8), "uint8"))
+
+
+# strings of a few families pass the 4-gram test by the million
+@pytest.mark.parametrize("length,families,k,filtered", [(64, 2, 6, False), (64, 8, 5, True), (100, 8, 6, False),
+                                                        (100, 400, 2, True), (64, 5000, 4, True)])
+def test_filter_leaves_related_strings(gpu, length, families, k, filtered):
+    q, c = _families(np.random.default_rng(families), 600, 20000, length, families, 0.02)
+    s = gpu.SearchBatch(q, c)
+    want = oracle.saturate(oracle.cross(q, c, k, threads=8), "uint8")
+    got, labels = _run(gpu, s, s.alloc("uint8"), k)
+    assert ("filter_pairs" in labels) == filtered, labels
+    np.testing.assert_array_equal(got, want)
+    qi, ci, d = s.matches(k)
+    wi, wj = np.nonzero(want <= k)
+    np.testing.assert_array_equal(qi, wi)
+    np.testing.assert_array_equal(ci, wj)
+    np.testing.assert_array_equal(d, want[wi, wj])
