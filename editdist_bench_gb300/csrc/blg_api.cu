@@ -211,6 +211,7 @@ struct blg_search {
     // and of the queries
     uint4 *ccnt = nullptr, *qcnt = nullptr;
     uint32_t *csig = nullptr, *qsig = nullptr;   // 4-gram signatures (blg_sig.cuh) of the same strings
+    void *csig_mem = nullptr;         // csig's own block (a large collection's; null csig: left out)
     void *sk_mem = nullptr;           // the queries' sketch block when this search owns it
     // choices in tile-transposed form (exact and unsorted runs), when the
     // padding to each tile's longest choice stays small
@@ -279,16 +280,55 @@ static cudaError_t launch_as(blg_ctx *c, const char *stage, const char *name, F 
     });
 }
 
+static void dev_free(blg_ctx *c, void *p) {
+    if (p) cudaFreeAsync(p, c->stream);
+}
+
+// Layouts that a search runs without, on the kernels that need none: the choices'
+// signatures of a large collection (32 bytes each), their order within tiles (2
+// bytes), a run's room for the deltas between stripes. Where the device has no room
+// for them they are left out, and where it runs full they are given back
+// (give_up_spares), so that no collection stops to fit for their sake. fault_alloc_after -2: every one fails, -3: the next other allocation
+// finds the device full once (tests).
+constexpr size_t kSpareBlock = size_t(64) << 20;          // smaller ones share a block with what they go with
+
+static void spare_alloc(blg_ctx *c, void **p, size_t bytes) {
+    *p = nullptr;
+    if (c->fault_alloc_after == -2 || cudaMallocAsync(p, bytes ? bytes : 16, c->stream) != cudaSuccess) {
+        cudaGetLastError();
+        *p = nullptr;
+    }
+}
+
+// The spares of the context's searches go back, in the stream's order: launches before
+// this one may still read them.
+static bool give_up_spares(blg_ctx *c) {
+    bool any = false;
+    for (blg_search *s : c->live) {
+        any |= s->csig_mem || s->tt_order;
+        dev_free(c, s->csig_mem);
+        if (s->csig_mem) s->csig = nullptr;
+        dev_free(c, s->tt_order);
+        s->csig_mem = nullptr;
+        s->tt_order = nullptr;
+    }
+    return any;
+}
+
 static cudaError_t dev_alloc(blg_ctx *c, void **p, size_t bytes) {
     if (c->fault_alloc_after >= 0 && c->fault_alloc_after-- == 0) {   // injected failure (tests)
         *p = nullptr;
         return cudaErrorMemoryAllocation;
     }
-    return cudaMallocAsync(p, bytes ? bytes : 16, c->stream);
-}
-
-static void dev_free(blg_ctx *c, void *p) {
-    if (p) cudaFreeAsync(p, c->stream);
+    const bool full = c->fault_alloc_after == -3;
+    if (full) c->fault_alloc_after = -1;
+    cudaError_t e = full ? cudaErrorMemoryAllocation : cudaMallocAsync(p, bytes ? bytes : 16, c->stream);
+    if (e == cudaErrorMemoryAllocation && give_up_spares(c)) {
+        cudaGetLastError();
+        cudaStreamSynchronize(c->stream);
+        e = cudaMallocAsync(p, bytes ? bytes : 16, c->stream);
+    }
+    return e;
 }
 
 static int check_offsets_host(blg_ctx *c, const int64_t *off, int64_t n) {
@@ -1365,6 +1405,7 @@ static int search_build_prefix(blg_ctx *c, const uint8_t *bc, const int64_t *oc,
 static int search_upload_choices(blg_ctx *c, const uint8_t *bc, const int64_t *oc, int64_t nc, blg_search *s,
                                  unsigned need = NEED_ALL, int32_t *perm_stage = nullptr) {
     s->nc = nc;
+    c->live.push_back(s);
     int rc = upload_strings(c, bc, oc, nc, s->c);
     if (rc) return rc;
     // Choices sorted by length (a stable counting sort on the host's thread
@@ -1387,8 +1428,9 @@ static int search_upload_choices(blg_ctx *c, const uint8_t *bc, const int64_t *o
             auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
             const size_t o_perm = 0, o_tab = up(sizeof(int32_t) * (size_t)nc),
                          o_soff = o_tab + up(sizeof(int64_t) * (size_t)(2 * n_len + 1)),
+                         sig = up(sizeof(uint32_t) * kSigWords * (size_t)nc),
                          o_csig = o_soff + up(sizeof(int64_t) * (size_t)(nc + 1)),
-                         o_ccnt = o_csig + up(sizeof(uint32_t) * kSigWords * (size_t)nc),
+                         o_ccnt = o_csig + (sig < kSpareBlock ? sig : 0),
                          o_buf = o_ccnt + up(sizeof(uint4) * (size_t)nc),
                          total = o_buf + (size_t)bytes + kSlackBefore + kSlackAfter;
             CK(dev_alloc(c, &s->sorted_mem, total), "cudaMallocAsync(sorted choices)");
@@ -1397,7 +1439,8 @@ static int search_upload_choices(blg_ctx *c, const uint8_t *bc, const int64_t *o
             s->lstart = (int64_t *)(m + o_tab);
             int64_t *d_bstart = s->lstart + (n_len + 1);
             int64_t *d_soff = (int64_t *)(m + o_soff);
-            s->csig = (uint32_t *)(m + o_csig);
+            if (sig >= kSpareBlock) spare_alloc(c, &s->csig_mem, sig);
+            s->csig = (uint32_t *)(sig >= kSpareBlock ? s->csig_mem : m + o_csig);
             s->ccnt = (uint4 *)(m + o_ccnt);
             uint8_t *d_buf = m + o_buf;
             CK(cudaMemcpyAsync(s->perm, perm, sizeof(int32_t) * nc, cudaMemcpyHostToDevice, c->stream), "H2D perm");
@@ -1461,8 +1504,7 @@ static int search_upload_choices(blg_ctx *c, const uint8_t *bc, const int64_t *o
                "cudaMallocAsync(tt)");
             CK(dev_alloc(c, (void **)&s->tt_base, sizeof(int64_t) * (size_t)(tiles + 1)), "cudaMallocAsync(tt base)");
             CK(dev_alloc(c, (void **)&s->tt_len, sizeof(int32_t) * (size_t)nc), "cudaMallocAsync(tt len)");
-            CK(dev_alloc(c, (void **)&s->tt_order, sizeof(uint16_t) * (size_t)tiles * kTileCands),
-               "cudaMallocAsync(tt order)");
+            spare_alloc(c, (void **)&s->tt_order, sizeof(uint16_t) * (size_t)tiles * kTileCands);
             CK(cudaMemcpyAsync(s->tt_base, base.data(), sizeof(int64_t) * (tiles + 1), cudaMemcpyHostToDevice,
                                c->stream), "H2D tt base");
             CK(launch(c, "transpose_choices", [&] {
@@ -1810,7 +1852,7 @@ static bool bits_faster(blg_ctx *c, const blg_search *s) {
 
 // Whether the bit-sliced kernel can run, and is the faster one, on the current classes.
 static bool bits_applies(blg_ctx *c, const blg_search *s) {
-    if (!s->tt || !s->bits_mem || c->tuning || bits_table_bytes(s->nsym, s->bits_longest) > kBitsMaxTable) return false;
+    if (!s->tt || !s->tt_order || !s->bits_mem || c->tuning || bits_table_bytes(s->nsym, s->bits_longest) > kBitsMaxTable) return false;
     const size_t scratch = s->bits_longest > 64 ? sizeof(uint32_t) * (size_t)bits_scratch_words(s->max_len) * (size_t)bits_warps(c->sms) : 0;
     return scratch <= kBitsMaxScratch && bits_faster(c, s);
 }
@@ -1879,7 +1921,7 @@ struct PassShare {
 static FilterPlan filter_plan(const blg_ctx *c, const blg_search *s, const SurvClasses &C, int k) {
     static const PassShare pass_share;
     FilterPlan f;
-    if (c->tuning || k > kSigMaxK || !s->csig || C.n == 0 || (double)s->nq * (double)s->nc < kFltMinPairs) return f;
+    if (c->tuning || k > kSigMaxK || !s->csig || !c->pl || C.n == 0 || (double)s->nq * (double)s->nc < kFltMinPairs) return f;
     std::vector<int32_t> len;
     for (auto &q : s->cls)
         if (!q.lanes) len.insert(len.end(), q.h_qlen.begin(), q.h_qlen.end());
@@ -1934,8 +1976,8 @@ static int search_run_bits(blg_ctx *c, blg_search *s, int dtype, void *d_out, bo
     void *scratch = nullptr;
     if (s->bits_longest > 64) {
         B.scratch_words = bits_scratch_words(s->max_len);
-        CK(dev_alloc(c, &scratch, sizeof(uint32_t) * (size_t)B.scratch_words * (size_t)bits_warps(c->sms)),
-           "cudaMallocAsync(stripe deltas)");
+        spare_alloc(c, &scratch, sizeof(uint32_t) * (size_t)B.scratch_words * (size_t)bits_warps(c->sms));
+        if (!scratch) return BLG_OK;
         B.scratch = (uint32_t *)scratch;
     }
     const cudaError_t e = launch(c, "search_bits", [&] {
@@ -2266,6 +2308,9 @@ static int search_matches_list(blg_ctx *c, blg_search *s, int k, blg_match *d_ou
 }
 
 static void search_release(blg_ctx *c, blg_search *s) {
+    c->live.erase(std::remove(c->live.begin(), c->live.end(), s), c->live.end());
+    dev_free(c, s->csig_mem);
+    s->csig_mem = nullptr;
     free_strings(c, s->q);
     free_strings(c, s->c);
     free_strings(c, s->cs);
@@ -3184,9 +3229,12 @@ int blg_init(int device, blg_ctx **out) {
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->rl_hdr, sizeof(unsigned long long) * (2 + (1u << 20)));
     if (e == cudaSuccess) c->rl_cap = 1u << 20;
     // the tensor-core filter's passers (32 MB): 2^22 pairs of a launch; more run
-    // the whole search in place
-    if (e == cudaSuccess) e = cudaMalloc((void **)&c->pl, sizeof(unsigned long long) * (4 + (1u << 22)));
-    if (e == cudaSuccess) c->pl_cap = 1u << 22;
+    // the whole search in place. A context does without it, and so without the filter
+    if (e == cudaSuccess && cudaMalloc((void **)&c->pl, sizeof(unsigned long long) * (4 + (1u << 22))) != cudaSuccess) {
+        cudaGetLastError();
+        c->pl = nullptr;
+    }
+    if (c->pl) c->pl_cap = 1u << 22;
     if (e == cudaSuccess) e = cudaEventCreate(&c->t0);
     if (e == cudaSuccess) e = cudaEventCreate(&c->t1);
     if (e == cudaSuccess) {
@@ -3866,7 +3914,7 @@ int blg_set_schedule(blg_ctx *c, int mode) {
 
 int blg_set_fault_injection(blg_ctx *c, int64_t alloc_fail_after, int32_t wait_polls) {
     ENTER(c);
-    c->fault_alloc_after = alloc_fail_after < 0 ? -1 : alloc_fail_after;
+    c->fault_alloc_after = alloc_fail_after < -3 ? -1 : alloc_fail_after;
     c->fault_wait_polls = wait_polls < 0 ? -1 : wait_polls;
     return BLG_OK;
 }

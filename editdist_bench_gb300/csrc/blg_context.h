@@ -52,7 +52,7 @@ struct blg_ctx {
     bool prof = false;
     // fault injection for tests of the error paths (blg_set_fault_injection):
     // the device allocation after `fault_alloc_after` more successes fails
-    // (-1: off); the short-pair tile kernel's first bounded copy wait and the
+    // (-1: off; -2, -3: spare_alloc in blg_api.cu); the short-pair tile kernel's first bounded copy wait and the
     // filter's waits between its warps give up after `fault_wait_polls` polls
     // (-1: the normal bound)
     int64_t fault_alloc_after = -1;
@@ -71,6 +71,7 @@ struct blg_ctx {
     // launch's gate, -], then pl_cap entries (allocated at init)
     unsigned long long *pl = nullptr;
     unsigned long long pl_cap = 0;
+    std::vector<struct blg_search *> live;   // searches that hold spare layouts (give_up_spares)
     size_t stage_bytes = 0;
     cudaEvent_t stage_done = nullptr;
     std::vector<ProfRec> prof_recs;

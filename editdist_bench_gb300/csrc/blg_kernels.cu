@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(256) k_prefix_text(DevStrings C, const int32_t
 // Transpose choices into tiles (see TransposedChoices); one thread per
 // (choice, word), bytes past a choice's end are zero.
 // order: the tile's positions by length, longest first, equal lengths in
-// place (a bitonic sort of length and position; tiles of one length skip it).
+// place (a bitonic sort of length and position; tiles of one length skip it). Null: no order.
 __global__ void __launch_bounds__(256) k_transpose_choices(DevStrings C, const int64_t *base, uint32_t *words,
                                                            int32_t *len, uint16_t *order, uint32_t *status) {
     __shared__ uint32_t s_key[kTileCands];
@@ -357,6 +357,7 @@ __global__ void __launch_bounds__(256) k_transpose_choices(DevStrings C, const i
             }
         }
         __syncthreads();
+        if (!order) continue;                                  // uniform
         bool mixed = false;
         for (int cl = threadIdx.x; cl < kTileCands; cl += blockDim.x)
             mixed |= s_key[cl] >> 31 == 0 && (s_key[cl] ^ s_key[0]) >> 10 != 0;

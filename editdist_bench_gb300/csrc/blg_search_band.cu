@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(256) k_sketch_strings(DevStrings S, const int3
         uint32_t v = my[lane];
         v |= __shfl_xor_sync(kFull, v, 8);
         v |= __shfl_xor_sync(kFull, v, 16);
-        if (lane < kSigWords) sig[i * kSigWords + lane] = v;
+        if (sig && lane < kSigWords) sig[i * kSigWords + lane] = v;
         if (lane == 0) counts[i] = make_uint4(t[0], t[1], t[2], t[3]);
         __syncwarp();
     }
@@ -241,7 +241,7 @@ cudaError_t launch_search_small(cudaStream_t st, const SurvClasses &C, const Dev
     return cudaGetLastError();
 }
 
-// perm null: S's strings in place, nothing copied.
+// perm null: S's strings in place, nothing copied. sig null: counts only.
 cudaError_t launch_sketch_strings(cudaStream_t st, int sms, const DevStrings &S, const int32_t *perm,
                                   const int64_t *dst_off, uint8_t *dst, uint32_t *sig, uint4 *counts,
                                   uint32_t *status) {

@@ -268,7 +268,10 @@ int blg_synchronize(blg_ctx *ctx);
  * failure (csrc/myers.c:162-164 returns -1, bench/cmyers.py:82-84 raises
  * MemoryError). alloc_fail_after >= 0: after that many more device
  * allocations of this context succeed, the next one fails as if the device
- * were out of memory (BLG_ERR_ALLOC); the hook is then spent. -1: off.
+ * were out of memory (BLG_ERR_ALLOC); the hook is then spent. -1: off. -2: the
+ * layouts that a search runs without (signatures of a large collection, the
+ * bit-sliced search's) find no room, until the hook is set again. -3: the next
+ * allocation finds the device full once, so such layouts are given back for it.
  * wait_polls >= 0: the short-pair tile kernel's bounded wait for its staged
  * strings, and the waits of the thresholded search's tensor-core filter, give
  * up after that many polls instead of their normal bound, so the call ends
