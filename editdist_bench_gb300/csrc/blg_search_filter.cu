@@ -454,15 +454,15 @@ __global__ void __launch_bounds__(kFltThreads, 1)
 // where the banded loop (survivor_warp) walks every column of a near-copy with
 // two scattered loads of the query's Peq rows, 32 lanes in 64 cache lines:
 // 52,000 passers of 100 to 256 bytes at k = 4 took 84 us that way and take 50.
-// The strings are first copied into shared memory; pairs longer than a slot
-// take the banded loop.
+// The strings are first copied into shared memory, whose slots hold the launch's
+// longest (sequential queries end at 512 bytes).
 // The filter leaves off filling the output when its tiles are done, long
 // before 1 GiB is written; here a third warp goes on with it, and as the fill
 // may pass an element after its result, results go to a list (list_emit) that
 // k_solve_finish stores. L.item null: the output is filled, results in place.
 constexpr int kLvThreads = 64;
 constexpr int kLvMaxK = kSigMaxK;
-constexpr int kLvMaxSlot = 1040;                         // bytes; longer strings take the banded loop
+constexpr int kLvMaxLength = 512;                        // of a query: 64 bytes of each of eight words
 
 // The repair launch's plan and its gate, by the blocks of a launch.
 __device__ __forceinline__ void repair_plan(const SurvClasses &C, const RepairPlan &R, int k) {
@@ -499,12 +499,13 @@ __global__ void __launch_bounds__(kLvThreads + 32)
          at += warps * 32) {
         bool live = at + lane < total;
         const uint8_t *a = Q.buf, *b = CS.buf;
-        int m = 0, n = 0, cls = 0, qi = 0;
+        int m = 0, n = 0;
         int64_t oidx = 0;
         if (live) {
             const unsigned long long e = P.item[at + lane];
             const int64_t sidx = (int64_t)(e & 0xffffffffu);
-            cls = seq_query(SC, (int)(e >> 32), qi);
+            int qi;
+            const int cls = seq_query(SC, (int)(e >> 32), qi);
             const int64_t row = __ldg(SC.cls[cls].qidx + qi);
             const uint4 cc = __ldg(ccnt + sidx);
             b = string_at(CS, sidx, n, status);
@@ -514,11 +515,10 @@ __global__ void __launch_bounds__(kLvThreads + 32)
             live = (n > m ? n - m : m - n) <= k && gram_dist(__ldg(qcnt + row), cc) <= 8u * (uint32_t)k;
         }
         const int sa = (int)(reinterpret_cast<uintptr_t>(a) & 15), sb = (int)(reinterpret_cast<uintptr_t>(b) & 15);
-        const bool fits = live && max(sa + m, sb + n) + 16 <= slot;
         // the lane's strings into its slots, 16 bytes at a time, all in flight at once (a lane's own copies: 24
         // instructions a warp for what shuffled addresses and whole lines took 1100)
         __syncwarp();
-        if (fits) {
+        if (live) {
             const uint32_t dst = smem_addr(slots + lane * slot);
             const uint8_t *pa = a - sa, *pb = b - sb;
             for (int x = 0; x < sa + m; x += 16)
@@ -528,19 +528,9 @@ __global__ void __launch_bounds__(kLvThreads + 32)
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
         if (!live) continue;
-        int d;
-        if (fits) {
-            const uint32_t base = (uint32_t)(warp * 64 + lane) * (uint32_t)slot;
-            const uint32_t *w = reinterpret_cast<const uint32_t *>(s_dyn);
-            d = furthest_distance<kLvThreads>(w, base + sa, m, w, base + 32 * slot + sb, n, k, f);
-        } else if (m == 0) {
-            d = n;
-        } else {
-            const SearchClass &cl = SC.cls[cls];
-            const uint64_t *peq = cl.peq + (size_t)qi * 256 * cl.nw;
-            const int nw = cl.nw;
-            d = band_distance(m, b, n, k, [&](uint32_t c, int p0) { return peq_window(peq + c * nw, nw, p0); }, Units{1u, 2u});
-        }
+        const uint32_t base = (uint32_t)(warp * 64 + lane) * (uint32_t)slot;
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(s_dyn);
+        const int d = furthest_distance<kLvThreads>(w, base + sa, m, w, base + 32 * slot + sb, n, k, f);
         if (d <= k) {
             if (L.item) list_emit(L, out, dtype, oidx, d);
             else store1(out, dtype, oidx, d);
@@ -600,9 +590,10 @@ cudaError_t launch_solve_passers(cudaStream_t st, int sms, const SurvClasses &C,
                                  int64_t longest, int k, int dtype, void *out, int64_t nc, const PasserList &P,
                                  const ResultList &L, const BatchFill &fill, const RepairPlan &plan, uint32_t *status) {
     if (C.n <= 0) return cudaSuccess;
-    if (k < 0 || k > kLvMaxK) return cudaErrorInvalidValue;
-    // a slot holds the launch's longest strings, an odd number of 16-byte banks
-    int slot = (int)std::min<int64_t>(kLvMaxSlot, longest + k + 15 + 16 + 15) & ~15;
+    if (k < 0 || k > kLvMaxK || longest > kLvMaxLength) return cudaErrorInvalidValue;
+    // a slot holds the launch's longest strings from any 16-byte boundary and octet's
+    // slack (a string up to k longer than its query), an odd number of 16-byte banks
+    int slot = (int)(longest + k + 15 + 16 + 15) & ~15;
     if (!(slot & 16)) slot += 16;
     const int smem = (kLvThreads / 32) * 64 * slot + (2 * k + 3) * kLvThreads * 2;
     cudaError_t e = cudaFuncSetAttribute(k_solve_passers, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

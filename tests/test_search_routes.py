@@ -46,3 +46,18 @@ def test_filter_leaves_related_strings(gpu, length, families, k, filtered):
     np.testing.assert_array_equal(qi, wi)
     np.testing.assert_array_equal(ci, wj)
     np.testing.assert_array_equal(d, want[wi, wj])
+
+
+def test_filter_longest_queries(gpu):
+    """Queries of 512 bytes, the most that a slot of the filter's solver holds, and
+    choices up to max_dist longer, starting at every byte of a 16-byte line."""
+    rng = np.random.default_rng(9)
+    q = W.random_strings(rng, rng.integers(509, 513, 130), TEXT)
+    c = W.concat(W.mutate(rng, W.take(q, rng.integers(0, 130, 2000)), rng.uniform(0, 0.012, 2000), TEXT),
+                 W.random_strings(rng, rng.integers(506, 516, 28000), TEXT))
+    c = W.take(c, rng.permutation(30000))
+    s = gpu.SearchBatch(q, c)
+    got, labels = _run(gpu, s, s.alloc("uint8"), 3)
+    assert "filter_pairs" in labels, labels
+    np.testing.assert_array_equal(got, oracle.saturate(oracle.cross(q, c, 3, threads=16), "uint8"))
+    assert set(np.unique(got)) == {0, 1, 2, 3, 4}
