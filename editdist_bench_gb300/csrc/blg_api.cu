@@ -781,13 +781,16 @@ static bool pairs_use_tile(const blg_ctx *c, const blg_pairs *p) {
 // chain run. With one pair in ten unrelated, DNA, then text: 250000 of 8 to 256 253 /
 // 352, 316 / 360; 70000 182 / 139, 193 / 140; 250000 of 4 to 80 77 / 88, 124 / 90; 70000
 // of 60 to 120 89 / 87, 100 / 89, of 200 to 400 269 / 434, 266 / 437; 20000 of 60 to 120
-// 102 / 66. What the sample may hold follows from these. A few that it does not show
+// 102 / 66. What the sample may hold follows from these. Texts' rows leave room for three
+// blocks on an SM, 116736 pairs: a second, emptier wave loses (132141 of 32 to 216 222 /
+// 211, 130000 of 64 65 / 58; 250000 of 64 86 / 86, of 60 to 120 146 / 168). A few that it does not show
 // cost as much: one in 100 of 20000 of 60 to 120 100 / 66, of 250000 texts of 4 to 80
 // 122 / 89.
 static bool pairs_use_bands(const blg_ctx *c, const blg_pairs *p) {
     if (c->sched != BLG_SCHED_AUTO || c->tuning || !p->trusted || p->too_long || p->cap[0] == 0 || p->nsym < 0) return false;
     if (p->n < kBandsMinPairs) return p->cap[1] == 0 && p->unrelated <= kPairSamples / 32;
-    const int64_t mean = p->len_max_side / p->n;
+    const int64_t mean = p->len_max_side / p->n, wave = (int64_t)c->sms * 3 * 256;
+    if (p->nsym > kBandSymbols && mean < 200 && p->n > wave && p->n < 200000) return false;
     int room = kPairSamples / 4;
     if (p->nsym > kBandSymbols) room = mean < 128 ? 0 : mean >= 200 ? room : p->n >= 200000 ? kPairSamples / 8 : 3;
     else if (mean >= 128 && mean < 200 && p->n < (1 << 17)) room = 1;

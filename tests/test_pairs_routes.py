@@ -62,7 +62,8 @@ def test_reach_leaves_what_it_would_slow_down(gpu, n, lo, hi, related, ks):
 
 # many pairs of another origin, or at most one in 50
 @pytest.mark.parametrize("n,share,alphabet,bands", [(20000, 0.25, W.DNA, False), (20000, 0.0, W.DNA, True), (70000, 0.5, W.DNA, False),
-                                                    (70000, 0.02, W.DNA, True), (70000, 0.1, TEXT, False), (70000, 0.0, TEXT, True)])
+                                                    (70000, 0.02, W.DNA, True), (70000, 0.1, TEXT, False), (70000, 0.0, TEXT, True),
+                                                    (120000, 0.0, TEXT, False), (120000, 0.0, W.DNA, True)])
 def test_bands_leave_mixed_sets(gpu, n, share, alphabet, bands):
     rng = np.random.default_rng(7)
     a, b = _near(rng, n, 60, 90, alphabet)
