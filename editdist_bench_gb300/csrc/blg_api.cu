@@ -2669,16 +2669,29 @@ static int batch_upload_body(blg_ctx *c, const blg_problem *pr, int nprob, blg_b
     BatchJob *jobs = (BatchJob *)hb(b_jobs);
     BatchFill *fills = (BatchFill *)hb(b_fills);
     // survivors per work unit: 1024 (the 256-problem batch 0.99 ms per step; 1.30
-    // with 4096), halved down to a warp's scan step of 128 while there would be
-    // fewer than 4 units per warp of the grid. Survivors estimated by lengths
-    // spread evenly over each problem's range.
-    double survivors = 0.0;
+    // with 4096), halved down to a warp's scan step of 128 while the survivors fill too
+    // few for the grid's warps: one a warp at max_dist up to 2, two up to 5, else four, as
+    // a survivor takes longer (units 1024, 512, 256, 128, microseconds: 12 x 200 x 30000
+    // related strings of 16 to 256, k = 2 327 253 211 193; 32 x 100 x 20000 reads of 64, k
+    // = 2 94 103 126 183; 64 x 300 x 10000 of 57 to 167, k = 2 62 62 67 76; 64 problems of
+    // all sizes, k up to 8, 217 at 512, 189 at 128).
+    double load = 0.0;                                    // survivors, as many as a warp's one unit may hold
     for (int i = 0; i < nprob; i++)
-        if (work[i] && eligible[i] && b->kk[i] >= 0 && b->kk[i] <= 31)
-            survivors += (double)pr[i].nq * (double)pr[i].nc *
-                         std::min(1.0, (2.0 * b->kk[i] + 1.0) / (double)(prep[i].mx - prep[i].mn + 1));
+        if (work[i] && eligible[i] && b->kk[i] >= 0 && b->kk[i] <= 31) {
+            const int64_t k = b->kk[i], qn = std::min<int64_t>(8, pr[i].nq), cn = std::min<int64_t>(16, pr[i].nc);
+            int64_t in = 0;                               // of a sample; lengths spread evenly at the least
+            for (int64_t x = 0; x < qn; x++)
+                for (int64_t y = 0; y < cn; y++) {
+                    const int64_t qi = pr[i].nq * x / qn, ci = pr[i].nc * y / cn;
+                    const int64_t gap = (pr[i].off_q[qi + 1] - pr[i].off_q[qi]) - (pr[i].off_c[ci + 1] - pr[i].off_c[ci]);
+                    in += gap <= k && gap >= -k;
+                }
+            const double even = std::min(1.0, (2.0 * (double)k + 1.0) / (double)(prep[i].mx - prep[i].mn + 1));
+            load += (double)pr[i].nq * (double)pr[i].nc * std::max(even, (double)in / (double)(qn * cn)) /
+                    (k <= 2 ? 1.0 : k <= 5 ? 2.0 : 4.0);
+        }
     int tile = 1024;
-    while (tile > 128 && survivors < 4.0 * c->sms * 4 * 8 * tile) tile >>= 1;
+    while (tile > 128 && load < (double)c->sms * 4 * 8 * tile) tile >>= 1;
     int nl = 0, nu = 0, nsk = 0, npq = 0, nj = 0, nf = 0, max_nwc = 1;
     lss_start[0] = ups_start[0] = sks_start[0] = pqs_start[0] = 0;
     // each group's first set of every kind

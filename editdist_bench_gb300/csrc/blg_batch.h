@@ -20,7 +20,7 @@ struct BatchJob {
     int64_t *tile_start;       // tile prefix per query (nq + 1)
     int64_t nc;
     int k, dtype, nw;
-    int tile;                  // survivors per work unit: 4096 (banded survivor jobs) or 1024
+    int tile;                  // survivors per work unit: 128 to 1024
     const uint4 *ccnt;         // binned 4-gram counts of the sorted choices
     const uint4 *qcnt;         // binned 4-gram counts of the queries (by query row)
     void *out;

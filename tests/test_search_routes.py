@@ -61,3 +61,14 @@ def test_filter_longest_queries(gpu):
     assert "filter_pairs" in labels, labels
     np.testing.assert_array_equal(got, oracle.saturate(oracle.cross(q, c, 3, threads=16), "uint8"))
     assert set(np.unique(got)) == {0, 1, 2, 3, 4}
+
+
+# work units of 1024, 512, 256 and 128 survivors, a last one partly full, beside an uneven problem
+@pytest.mark.parametrize("nq,nc", [(400, 13007), (300, 10001), (100, 15003), (10, 2005)])
+def test_batch_unit_sizes(gpu, nq, nc):
+    rng = np.random.default_rng(nq)
+    probs = [_sets(rng, nq, nc, 64, 64, W.DNA) + (2, "uint8"), _sets(rng, 3, 701, 10, 90, TEXT) + (7, "uint16")]
+    b = gpu.ProblemBatch(probs)
+    for rep in range(2):
+        for got, (q, c, k, dt) in zip([o.get() for o in b.run()], probs):
+            np.testing.assert_array_equal(got, oracle.saturate(oracle.cross(q, c, k, threads=16), dt))
