@@ -1146,16 +1146,22 @@ static int bits_build(blg_ctx *c, const std::vector<QueryClass> &qc, blg_search 
     return BLG_OK;                                       // (pageable: the copy completed before return)
 }
 
+static std::array<uint8_t, 256> bytes_of(const uint8_t *p, int64_t n) {
+    std::array<uint8_t, 256> any{};                        // (a local: a store into it cannot move `p`)
+    for (int64_t x = 0; x < n; x++) any[p[x]] = 1;
+    return any;
+}
+
 // The distinct bytes of queries [0, nq): symbols 1 .. nsym in byte order; the
 // bytes of no query map to symbol 0, an empty row of the kernel's table.
 static void query_symbols(const uint8_t *bq, const int64_t *oq, int64_t nq, blg_search *s) {
     HostPool &pool = HostPool::get();
     const int64_t lo = oq[0], bytes = oq[nq] - lo;
-    const int nt = bytes >= (1 << 18) ? pool.size() : 1;
+    const int nt = (int)std::max<int64_t>(1, std::min<int64_t>(pool.size(), bytes >> 16));
     std::vector<std::array<uint8_t, 256>> seen((size_t)nt);
     pool.run(nt, [&](int t) {
-        seen[t].fill(0);
-        for (int64_t x = lo + bytes * t / nt, e = lo + bytes * (t + 1) / nt; x < e; x++) seen[t][bq[x]] = 1;
+        const int64_t x = bytes * t / nt;
+        seen[t] = bytes_of(bq + lo + x, bytes * (t + 1) / nt - x);
     });
     std::array<uint8_t, 256> any{};
     for (auto &v : seen)
@@ -1569,7 +1575,7 @@ static int search_upload_queries(blg_ctx *c, const uint8_t *bq, const int64_t *o
 // string stand for it. Host work beside the choices' upload.
 static void sample_grams(const uint8_t *bq, const int64_t *oq, int64_t nq, const uint8_t *bc, const int64_t *oc, int64_t nc,
                          blg_search *s) {
-    if (!s->csig || (double)nq * (double)nc < kFltMinPairs) return;
+    if (!s->csig || (double)nq * (double)nc < 1.5 * kFltMinPairs) return;   // (search_small takes what is smaller)
     struct Sig {
         uint64_t w[kSigWords / 2] = {};
     };
