@@ -274,6 +274,10 @@ class SearchBench:
             return OPS_PER_WORD32_STEP * words * float(np.diff(self.w.c[1]).sum())
         return None if exit_cols_sum is None else OPS_PER_WORD32_STEP * exit_cols_sum
 
+    def bit_sliced_ops(self) -> float:
+        """ALU operations of the bit-sliced search: four per matrix cell of 32 queries."""
+        return 4.0 / 32.0 * float(np.diff(self.w.q[1]).sum()) * float(np.diff(self.w.c[1]).sum())
+
     def alg_bytes(self, i=0):
         return self.pairs * np.dtype(self.runs[i][1]).itemsize + float(self.w.q[1][-1] + self.w.c[1][-1])
 
@@ -709,19 +713,31 @@ def roofline_block(bench, kstats, top, peak, exit_sum, dev, clock_mhz) -> dict:
     """The dominant launch label's roofline: algorithmic bytes and integer
     ops per step over its event time (HBM and integer-pipe fractions, the
     binding one first), plus its issue-slot utilisation from the warp
-    instructions per pair its ncu summary records."""
+    instructions per pair its ncu summary records. The integer ops are those of
+    the kernel's own method where it is bit-sliced, else the reference's column
+    loop over the columns its exit rule processes; a run that filters most of
+    those columns away, or walks furthest-reaching points instead, has no integer
+    fraction against them and is held to HBM. The bytes are the whole step's, so
+    their rate is over all its launches."""
     ms = kstats[top]["ms_per_step"]
-    ops = bench.alg_ops(0, exit_sum)
+    # (pairs_reach is a second label of the pairs_solve launch)
+    step_ms = sum(v["ms_per_step"] for n, v in kstats.items() if n != "pairs_reach")
+    sliced, reach = top == "search_bits", "pairs_reach" in kstats
+    ops = bench.bit_sliced_ops() if sliced else bench.alg_ops(0, exit_sum)
     hpeak, hsrc = hbm_peak()
-    hbm = {"achieved": bench.alg_bytes(0) / (ms / 1e3) / 1e9, "peak": hpeak, "unit": "GB/s",
+    hbm = {"achieved": bench.alg_bytes(0) / (step_ms / 1e3) / 1e9, "peak": hpeak, "unit": "GB/s",
            "peak_source": hsrc, "alg_bytes_per_step": bench.alg_bytes(0)}
     hbm["frac"] = hbm["achieved"] / hpeak
     ipart = {"peak": peak.get("gops"), "unit": "Gop/s",
              "peak_source": "measured: libblg_probe LOP3/IADD3 stream on this GPU", "peak_detail": peak}
     if ops is not None and peak.get("gops"):
-        ipart["alg_ops_per_step"] = ops
-        ipart["achieved"] = ops / (ms / 1e3) / 1e9
-        ipart["frac"] = ipart["achieved"] / peak["gops"]
+        rate = ops / (ms / 1e3) / 1e9
+        if sliced or (rate <= peak["gops"] and not reach):
+            ipart.update({"alg_ops_per_step": ops, "achieved": rate, "frac": rate / peak["gops"],
+                          "ops": "bit-sliced cells" if sliced else "reference's word steps"})
+        else:
+            ipart.update({"reference_ops_per_step": ops, "achieved": None, "frac": None,
+                          "ops": "the reference's word steps, which this run does not take"})
     prof = read_profile(top, bench.w.name)
     issue = None
     if prof.get("inst_per_unit") and dev.get("sms"):
@@ -734,8 +750,9 @@ def roofline_block(bench, kstats, top, peak, exit_sum, dev, clock_mhz) -> dict:
                  "time_share": share, "source": prof["path"],
                  "how": "inst_per_unit x pairs per step / (event ms x time_share x SMs x 4 issue slots per clock "
                         "x SM clock)"}
-    # short exact pairs (config 1) are bound by moving their bytes; the rest by the integer pipe
-    primary = hbm if (bench.kind == "pairwise" and bench.runs[0][0] is None) else ipart
+    # short exact pairs (config 1) are bound by moving their bytes, and runs that do not
+    # take the reference's steps are held to that; the rest by the integer pipe
+    primary = hbm if (bench.kind == "pairwise" and bench.runs[0][0] is None) or (ops and ipart.get("frac") is None) else ipart
     traffic = prof.get("traffic_bytes_per_launch")
     launches = kstats[top]["launches"]
     return {"kernel": top, "bound": "hbm" if primary is hbm else "int", "achieved": primary.get("achieved"),
