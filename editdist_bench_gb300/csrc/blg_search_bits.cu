@@ -11,8 +11,8 @@
 //    character picks the symbol's rows and the column walks down them with
 //    16-byte loads at constant offsets. Symbols lie `stride` words apart, 4 mod
 //    32, so eight different symbols at one row hit different banks.
-//  * The vertical deltas of 64 rows stay in registers (128 of them; 168 per
-//    thread, 12 warps per SM). Longer queries run stripe by stripe: the
+//  * The vertical deltas of 64 rows stay in registers (128 of them; 231 per
+//    thread, 8 warps per SM). Longer queries run stripe by stripe: the
 //    horizontal deltas leaving a stripe's bottom row, two words per column,
 //    pass through a per-warp scratch row in global memory that L2 holds.
 //  * The last stripe has as many rows as the group's longest query needs (a
