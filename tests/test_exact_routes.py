@@ -55,3 +55,18 @@ def test_chunks_of_a_larger_search(gpu):
     assert "search_bits" in labels and "search_pfx" not in labels, labels
     rows = np.arange(0, 400, 37)
     np.testing.assert_array_equal(got[0][rows], oracle.saturate(oracle.cross(W.take(q, rows), c, threads=8), "uint16"))
+
+
+# choices that share most of their columns, queries past the prefix kernel's two words
+# alone and beside short ones
+@pytest.mark.parametrize("nq,lo,hi", [(300, 150, 256), (300, 129, 129), (300, 60, 256), (300, 64, 128)])
+def test_long_queries_beside_shared_prefixes(gpu, nq, lo, hi):
+    rng = np.random.default_rng(lo)
+    q = W.random_strings(rng, rng.integers(lo, hi + 1, nq))
+    c, off = W.random_strings(rng, np.full(9001, 64))
+    c.reshape(-1, 64)[:, :48] = rng.choice(W.DNA, (40, 48))[rng.integers(0, 40, 9001)]
+    labels = _run(gpu, q, (c, off))
+    if lo > 128:
+        assert "search_bits" in labels and "search_pfx" not in labels, labels
+    if hi <= 128:
+        assert "search_pfx" in labels and "search_bits" not in labels, labels
