@@ -123,7 +123,7 @@ constexpr size_t kBitsMaxTable = 160 << 10;
 constexpr size_t kBitsMaxScratch = size_t(512) << 20;
 // The prefix-reuse kernel where the restarts skip enough of the text (it takes
 // 16.3 ms on 4096 x 65536 reads of 64 bases with none skipped, the bit-sliced
-// one 9.2). Searches of 33 to 64 queries of at most two words take it too,
+// one 9.2). Resident searches of 33 to 64 queries of at most two words take it too,
 // which is the slower side (64 x 20000 reads of 64: 186 us against 77; 64 x
 // 65536: 498 against 183): tests/test_gpu_prefix.py expects this kernel there.
 constexpr double kBitsPfxSaving = 0.45;
@@ -1260,24 +1260,37 @@ enum { NEED_SORTED = 1, NEED_TT = 2, NEED_PFX = 4, NEED_ALL = 7 };
 constexpr int64_t kPfxMinChoices = 4096;
 constexpr double kPfxMinSaving = 0.02;
 
-// The share of the text that sorted neighbours have in common, from 2048
+// A choice's first 16 bytes as two big-endian words, zeros past its end.
+struct PrefixKey {
+    uint64_t hi, lo;
+    int32_t idx;
+    bool operator<(const PrefixKey &o) const { return hi != o.hi ? hi < o.hi : lo < o.lo; }
+};
+
+static PrefixKey prefix_key(const uint8_t *bc, const int64_t *oc, int64_t i) {
+    const uint8_t *p = bc + oc[i];
+    const int64_t len = oc[i + 1] - oc[i];
+    uint64_t w[2] = {0, 0};
+    for (int b = 0; b < 16; b++) w[b >> 3] = w[b >> 3] << 8 | (b < len ? p[b] : 0u);
+    return {w[0], w[1], (int32_t)i};
+}
+
+// The share of the text that sorted neighbours have in common, from up to 2048
 // choices spread over the set: a set whose restarts would skip half of its
-// columns shows most of that in a sample.
-static double sampled_prefix_share(const uint8_t *bc, const int64_t *oc, int64_t nc) {
-    const int64_t n = std::min<int64_t>(nc, 2048);
-    std::vector<int64_t> at((size_t)n);
-    for (int64_t i = 0; i < n; i++) at[i] = nc * i / n;
-    std::sort(at.begin(), at.end(), [&](int64_t x, int64_t y) {
-        return std::lexicographical_compare(bc + oc[x], bc + oc[x + 1], bc + oc[y], bc + oc[y + 1]);
-    });
+// columns shows most of that in a sample. Some 0.1 us a choice.
+static double sampled_prefix_share(const uint8_t *bc, const int64_t *oc, int64_t nc, int64_t n = 2048) {
+    n = std::min(nc, n);
+    std::vector<PrefixKey> at((size_t)n);
+    for (int64_t i = 0; i < n; i++) at[i] = prefix_key(bc, oc, nc * i / n);
+    std::sort(at.begin(), at.end());
     int64_t same = 0, all = 0;
     for (int64_t i = 1; i < n; i++) {
-        const uint8_t *x = bc + oc[at[i - 1]], *y = bc + oc[at[i]];
-        const int64_t lim = std::min(oc[at[i - 1] + 1] - oc[at[i - 1]], oc[at[i] + 1] - oc[at[i]]);
+        const int64_t a = at[i - 1].idx, b = at[i].idx;
+        const int64_t lim = std::min(oc[a + 1] - oc[a], oc[b + 1] - oc[b]);
         int64_t l = 0;
-        while (l < lim && x[l] == y[l]) l++;
+        while (l < lim && bc[oc[a] + l] == bc[oc[b] + l]) l++;
         same += l;
-        all += oc[at[i] + 1] - oc[at[i]];
+        all += oc[b + 1] - oc[b];
     }
     return all > 0 ? (double)same / (double)all : 0.0;
 }
@@ -1307,33 +1320,19 @@ static int search_build_prefix(blg_ctx *c, const uint8_t *bc, const int64_t *oc,
         }
     }
     if (sym.empty() || (int)sym.size() > kPfxMaxSymbols) return BLG_OK;
-    struct Key {
-        uint64_t hi, lo;
-        int32_t idx;
-    };
-    std::vector<Key> keys((size_t)nc);
-    auto be8 = [](const uint8_t *p, int64_t len, int64_t from) {
-        uint64_t v = 0;
-        for (int b = 0; b < 8; b++) v = (v << 8) | (from + b < len ? p[from + b] : 0u);
-        return v;
-    };
-    auto less = [](const Key &a, const Key &b) { return a.hi != b.hi ? a.hi < b.hi : a.lo < b.lo; };
+    std::vector<PrefixKey> keys((size_t)nc);
     pool.run(nt, [&](int t) {
-        for (int64_t i = cut[t]; i < cut[t + 1]; i++) {
-            const uint8_t *p = bc + oc[i];
-            const int64_t len = oc[i + 1] - oc[i];
-            keys[i] = Key{be8(p, len, 0), be8(p, len, 8), (int32_t)i};
-        }
-        std::sort(keys.begin() + cut[t], keys.begin() + cut[t + 1], less);
+        for (int64_t i = cut[t]; i < cut[t + 1]; i++) keys[i] = prefix_key(bc, oc, i);
+        std::sort(keys.begin() + cut[t], keys.begin() + cut[t + 1]);
     });
-    std::vector<Key> tmp((size_t)nc);
+    std::vector<PrefixKey> tmp((size_t)nc);
     for (int w = 1; w < nt; w *= 2) {                        // merge sorted runs pairwise, in parallel
         const int groups = (nt + 2 * w - 1) / (2 * w);
         pool.run(groups, [&](int g) {
             const int64_t lo = cut[std::min(nt, 2 * g * w)], mid = cut[std::min(nt, 2 * g * w + w)],
                           hi = cut[std::min(nt, 2 * g * w + 2 * w)];
             std::merge(keys.begin() + lo, keys.begin() + mid, keys.begin() + mid, keys.begin() + hi,
-                       tmp.begin() + lo, less);
+                       tmp.begin() + lo);
         });
         keys.swap(tmp);
     }
@@ -1534,6 +1533,7 @@ static int search_upload_choices(blg_ctx *c, const uint8_t *bc, const int64_t *o
 static int search_run(blg_ctx *c, blg_search *s, int k, int dtype, void *d_out, int64_t q0 = 0,
                       int64_t q1 = -1);
 static bool bits_applies(blg_ctx *c, const blg_search *s);
+static bool prefix_pays(blg_ctx *c, const blg_search *s, const uint8_t *bc, const int64_t *oc, int64_t nc);
 
 // As many equally frequent bytes as repeat as often as a sample's bytes do (DNA with
 // a rare N: 4), from up to 64 pieces of 64 bytes.
@@ -1795,15 +1795,20 @@ static int64_t class_queries(const blg_search *s) {
     return n;
 }
 
+// A search of 33 to 64 queries, all of one or two words. A chunk of a larger search
+// (cdist_pipelined) is none.
+static bool held_to_prefix(const blg_search *s) {
+    return s->bits_nq >= kPfxMinQueries && s->bits_nq <= kPfxMaxQueries && s->bits_longest <= 128 &&
+           class_queries(s) == s->nq;
+}
+
 // Whether the exact run of the sequential classes takes the prefix-reuse kernel
 // whatever the others' estimates: queries of one and two words alone, which it takes
 // all. With longer ones beside them the estimates decide (20000 choices of 200 that
 // share 70%, 300 queries of 150 to 256: 4751 us word by word, 2619 bit-sliced; of 60 to
-// 256, some of them by prefixes: 3648, 2187). A chunk of a larger search (cdist_pipelined)
-// is no search of 33 to 64 queries.
+// 256, some of them by prefixes: 3648, 2187).
 static bool use_prefix(const blg_search *s) {
-    const bool held = s->bits_nq >= kPfxMinQueries && s->bits_nq <= kPfxMaxQueries && class_queries(s) == s->nq;
-    return s->pfx && (s->bits_nq == 0 || (s->bits_longest <= 128 && (held || s->pfx_saving >= kBitsPfxSaving)));
+    return s->pfx && (s->bits_nq == 0 || held_to_prefix(s) || (s->bits_longest <= 128 && s->pfx_saving >= kBitsPfxSaving));
 }
 
 // Estimated microseconds of an exact run, by kernel: each has a floor, the time of
@@ -1825,9 +1830,9 @@ static double word_us(blg_ctx *c, const blg_search *s, const blg_search::Cls &k)
 
 // The prefix-reuse kernel's lanes hold queries, 128 of one word or 64 of two to a
 // warp, real or not. 500 x 20000 reads of 64: 668 (621 measured); 1 x 20000: 206 (185).
-static double prefix_us(const blg_search *s, const blg_search::Cls &k) {
+static double prefix_us(const blg_search *s, const blg_search::Cls &k, double saving) {
     const double cols = (double)s->max_len, avg = (double)s->c.d.bytes / (double)s->nc, slots = k.nw == 1 ? 128.0 : 64.0;
-    const double rate = 1.1e-6 * (1.0 - s->pfx_saving) * avg * k.nw * std::ceil(k.nq / slots) * slots * (double)s->nc;
+    const double rate = 1.1e-6 * (1.0 - saving) * avg * k.nw * std::ceil(k.nq / slots) * slots * (double)s->nc;
     return 5.0 + std::max(1.6 * cols, 0.6 * cols + rate);
 }
 
@@ -1836,17 +1841,16 @@ static double prefix_us(const blg_search *s, const blg_search::Cls &k) {
 // 256: 157 against 1180; 100 x 5000 reads of 64: 165 against 104).
 static bool class_prefix(blg_ctx *c, const blg_search *s, const blg_search::Cls &k) {
     if (!s->pfx || !search_pfx_supported(k.nw)) return false;
-    return use_prefix(s) || c->tuning || word_us(c, s, k) >= 0.8 * prefix_us(s, k);
+    return use_prefix(s) || c->tuning || word_us(c, s, k) >= 0.8 * prefix_us(s, k, s->pfx_saving);
 }
 
-// Whether the bit-sliced kernel beats the others on an exact run. A unit takes 6.6
-// ns per cell of its 32 x 32 pairs alone on its SM partition and 1.6 times that with
+// The bit-sliced kernel: a unit takes 6.6 ns per cell of its 32 x 32 pairs alone on its SM partition and 1.6 times that with
 // a second one beside it, two rounds over the eight warps of an SM cost twice, and a
 // CTA with units of two groups waits for the last of the first. Before the last
 // round, shorter choices and groups count as such. 33 x 65536 reads of 256: 2.7 ms
 // (2.8 measured, 2.3 of the word kernel); 4 x 40000 of 16 to 256: 0.81 (0.85, 0.51);
 // 32 x 20000 of 64: 51 us (52, 206); 1000 x 20000: 735 (767, 1386).
-static bool bits_faster(blg_ctx *c, const blg_search *s) {
+static double bits_us(blg_ctx *c, const blg_search *s) {
     const double cols = (double)s->max_len, avg = (double)s->c.d.bytes / (double)s->nc;
     const int64_t groups = (s->bits_nq + 31) / 32, units = groups * ((s->nc + 31) / 32), slots = bits_warps(c->sms);
     const double alone = 6.6e-3 * cols * (double)std::max(8, (s->bits_longest + 7) & ~7);
@@ -1854,11 +1858,15 @@ static bool bits_faster(blg_ctx *c, const blg_search *s) {
     double rounds = 1.6 * full * (cols > 0.0 ? avg / cols : 1.0) * s->bits_share;
     rounds += rem == 0.0 ? 0.0 : 2.0 * rem <= (double)slots ? 1.0 : 1.6;
     if (groups > 1 && full > 0.0) rounds += 0.3;
-    const double bits = 8.0 + alone * std::max(1.0, rounds);
+    return 8.0 + alone * std::max(1.0, rounds);
+}
+
+// Whether it beats the others on an exact run.
+static bool bits_faster(blg_ctx *c, const blg_search *s) {
     double other = 0.0;
     for (auto &k : s->cls)
-        if (!k.lanes) other += class_prefix(c, s, k) ? prefix_us(s, k) : word_us(c, s, k);
-    return bits <= 1.05 * other;
+        if (!k.lanes) other += class_prefix(c, s, k) ? prefix_us(s, k, s->pfx_saving) : word_us(c, s, k);
+    return bits_us(c, s) <= 1.05 * other;
 }
 
 // Whether the bit-sliced kernel can run, and is the faster one, on the current classes.
@@ -1866,6 +1874,33 @@ static bool bits_applies(blg_ctx *c, const blg_search *s) {
     if (!s->tt || !s->tt_order || !s->bits_mem || c->tuning || bits_table_bytes(s->nsym, s->bits_longest) > kBitsMaxTable) return false;
     const size_t scratch = s->bits_longest > 64 ? sizeof(uint32_t) * (size_t)bits_scratch_words(s->max_len) * (size_t)bits_warps(c->sms) : 0;
     return scratch <= kBitsMaxScratch && bits_faster(c, s);
+}
+
+// Whether a one-call exact search sorts its choices for the prefix-reuse kernel, which
+// nothing hides there: where the kernels without that layout take a fourth longer than
+// with it and the sort (0.033 us a choice with a pool of 16 threads: 5000 to 65536
+// choices of 12 to 256 bytes), judged by a sample that takes a fortieth of their time.
+// Whole calls with uint8 results, sorting always / by this rule, microseconds: 16 x 8000
+// of 3 to 40 bytes 416 / 118, 200 x 20000 reads of 64 1130 / 350, 4 x 65536 of 16 to 256
+// 3700 / 700, 40 x 20000 reads of 64 1090 / 207; with 70% of the columns shared 300 x
+// 30000 1590 / 566, 4000 x 16000 3815 / 3470, 2000 x 4200 of 100 to 128 1698 / 1418.
+static bool prefix_pays(blg_ctx *c, const blg_search *s, const uint8_t *bc, const int64_t *oc, int64_t nc) {
+    if (nc < kPfxMinChoices || nc >= INT32_MAX) return false;
+    const double sort_us = 0.033 * (double)nc;
+    const bool bits = bits_applies(c, s);
+    auto words_us = [&](double saving) {               // saving < 0: no such layout
+        double us = 0.0;
+        for (auto &k : s->cls) {
+            if (k.lanes) continue;
+            const double word = word_us(c, s, k);
+            us += saving >= 0.0 && search_pfx_supported(k.nw) ? std::min(word, prefix_us(s, k, saving)) : word;
+        }
+        return us;
+    };
+    const double now = bits ? bits_us(c, s) : words_us(-1.0);
+    if (now <= 1.2 * sort_us) return false;
+    const double share = sampled_prefix_share(bc, oc, nc, (int64_t)std::max(256.0, std::min(1024.0, now / 4)));
+    return (!bits || share >= 0.7 * kBitsPfxSaving) && words_us(share) + sort_us < 0.8 * now;
 }
 
 // Whether a thresholded run of the sequential classes filters on the tensor
@@ -3639,7 +3674,8 @@ int blg_cdist(blg_ctx *c, const uint8_t *bq, const int64_t *oq, int64_t nq, cons
         const bool pipe = !out_device && nq >= 2 && obytes >= (u4 ? (32u << 20) : (64u << 20));
         if (!pipe) {
             const bool surv = max_dist >= 0 && c->sched != BLG_SCHED_PLAIN;
-            rc = search_upload(c, bq, oq, nq, bc, oc, nc, &s, surv ? NEED_SORTED | NEED_TT : NEED_TT | NEED_PFX);
+            rc = search_upload(c, bq, oq, nq, bc, oc, nc, &s, surv ? NEED_SORTED | NEED_TT : NEED_TT);
+            if (!rc && max_dist < 0 && prefix_pays(c, &s, bc, oc, nc)) rc = search_build_prefix(c, bc, oc, nc, &s);
             if (!rc) rc = search_run(c, &s, max_dist, u4 ? BLG_UINT8 : dtype, u4 ? d8 : d_out);
             if (!rc && u4) rc = pack_u4(c, d8, 0, n, d_out);
             if (!rc && !out_device) {

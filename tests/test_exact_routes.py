@@ -70,3 +70,21 @@ def test_long_queries_beside_shared_prefixes(gpu, nq, lo, hi):
         assert "search_bits" in labels and "search_pfx" not in labels, labels
     if hi <= 128:
         assert "search_pfx" in labels and "search_bits" not in labels, labels
+
+
+# one call: the choices are sorted only where that takes less than it saves
+@pytest.mark.parametrize("nq,nc,stem,symbols,pfx", [(100, 8001, 0, 4, False), (100, 8001, 48, 4, False), (64, 8001, 0, 4, False),
+                                                    (4000, 8001, 60, 4, True), (4000, 8001, 0, 4, False),
+                                                    (300, 8001, 48, 250, True), (2000, 8001, 48, 250, True)])
+def test_one_call_sorts_where_it_pays(gpu, nq, nc, stem, symbols, pfx):
+    rng = np.random.default_rng(nq + stem)
+    q = W.random_strings(rng, rng.integers(100, 129, nq), np.arange(symbols, dtype=np.uint8) if symbols > 4 else W.DNA)
+    if symbols > 4:                                # a table too large for the bit-sliced kernel
+        q = W.concat(q, W.random_strings(rng, [512], np.arange(symbols, dtype=np.uint8)))
+    c, off = W.random_strings(rng, np.full(nc, 64))
+    c.reshape(-1, 64)[:, :stem] = rng.choice(W.DNA, (40, stem))[rng.integers(0, 40, nc)]
+    got = []
+    labels = _labels(_lib.context(), lambda: got.append(gpu.cdist_packed(q, (c, off), dtype="uint8")))
+    assert ("search_pfx" in labels) == ("prefix_text" in labels) == pfx, labels
+    rows = np.unique(np.append(np.arange(0, nq, 1 + nq // 40), len(q[1]) - 2))
+    np.testing.assert_array_equal(got[0][rows], oracle.saturate(oracle.cross(W.take(q, rows), (c, off), threads=8), "uint8"))
