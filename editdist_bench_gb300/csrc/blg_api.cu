@@ -1844,12 +1844,13 @@ static bool class_prefix(blg_ctx *c, const blg_search *s, const blg_search::Cls 
     return use_prefix(s) || c->tuning || word_us(c, s, k) >= 0.8 * prefix_us(s, k, s->pfx_saving);
 }
 
-// The bit-sliced kernel: a unit takes 6.6 ns per cell of its 32 x 32 pairs alone on its SM partition and 1.6 times that with
-// a second one beside it, two rounds over the eight warps of an SM cost twice, and a
-// CTA with units of two groups waits for the last of the first. Before the last
-// round, shorter choices and groups count as such. 33 x 65536 reads of 256: 2.7 ms
-// (2.8 measured, 2.3 of the word kernel); 4 x 40000 of 16 to 256: 0.81 (0.85, 0.51);
-// 32 x 20000 of 64: 51 us (52, 206); 1000 x 20000: 735 (767, 1386).
+// The bit-sliced kernel: a unit takes 6.6 ns per cell of its 32 x 32 pairs alone on
+// its SM partition and 1.6 times that with a second one beside it, two rounds over the
+// eight warps of an SM cost twice, and a CTA with units of two groups waits for the
+// last of the first. Before the last round, shorter choices and groups count as such.
+// 33 x 65536 reads of 256: 2.7 ms (2.8 measured, 2.3 of the word kernel); 4 x 40000 of
+// 16 to 256: 0.81 (0.85, 0.51); 32 x 20000 of 64: 51 us (52, 206); 1000 x 20000: 735
+// (767, 1386).
 static double bits_us(blg_ctx *c, const blg_search *s) {
     const double cols = (double)s->max_len, avg = (double)s->c.d.bytes / (double)s->nc;
     const int64_t groups = (s->bits_nq + 31) / 32, units = groups * ((s->nc + 31) / 32), slots = bits_warps(c->sms);
