@@ -230,7 +230,9 @@ struct blg_search {
     int64_t max_len = 0;              // longest choice
     double warp_len = 0.0;            // mean of the longest of 32 neighbours
     int gram_sym = 256;              // the queries' bytes, as that many equally frequent ones (filter_plan)
-    float gram_pass[kSigMaxK + 1] = {};   // by k: share of a sample's pairs whose 4-grams allow it (sample_grams)
+    // by k: share of a sample's pairs whose 4-grams allow it, and of those the ones whose
+    // lengths do (sample_grams)
+    float gram_pass[kSigMaxK + 1] = {}, gram_near[kSigMaxK + 1] = {};
     // exact runs, bit-sliced over the queries (k_search_bits): the distinct
     // bytes of the queries (nsym 0: not counted, or too many) and, per class set, the
     // sequential queries by length
@@ -1571,45 +1573,51 @@ static int search_upload_queries(blg_ctx *c, const uint8_t *bq, const int64_t *o
 }
 
 // Of 32 queries x 64 choices spread over the sets, the share whose signatures differ
-// by at most 8 k, for every k of the filter (filter_plan). The first 512 bytes of a
-// string stand for it. Host work beside the choices' upload.
+// by at most 8 k, and whose lengths by at most k beside that, for every k of the filter
+// (filter_plan). The first 512 bytes of a string stand for it. Host work
+// beside the choices' upload. (The bins as they are hashed: sig_bit's places give the same counts.)
 static void sample_grams(const uint8_t *bq, const int64_t *oq, int64_t nq, const uint8_t *bc, const int64_t *oc, int64_t nc,
                          blg_search *s) {
     if (!s->csig || (double)nq * (double)nc < 1.5 * kFltMinPairs) return;   // (search_small takes what is smaller)
     struct Sig {
-        uint64_t w[kSigWords / 2] = {};
+        uint64_t w[4] = {};
     };
     auto signature = [](const uint8_t *p, int64_t len) {
         Sig g;
-        uint32_t gram = 0;
-        for (int64_t i = 0; i < std::min<int64_t>(512, len); i++) {
+        len = std::min<int64_t>(512, len);
+        uint32_t gram = len >= 3 ? (uint32_t)p[0] << 16 | (uint32_t)p[1] << 8 | p[2] : 0;
+        for (int64_t i = 3; i < len; i++) {
             gram = gram << 8 | p[i];
-            if (i < 3) continue;
-            const uint32_t bit = sig_bit(gram);
-            g.w[bit >> 6] |= 1ull << (bit & 63);
+            const uint32_t bin = sig_bin(gram);
+            g.w[bin >> 6] |= 1ull << (bin & 63);
         }
         return g;
     };
     const int64_t qn = std::min<int64_t>(32, nq), cn = std::min<int64_t>(64, nc);
     Sig q[32];
-    for (int64_t x = 0; x < qn; x++) q[x] = signature(bq + oq[nq * x / qn], oq[nq * x / qn + 1] - oq[nq * x / qn]);
-    int count[kSigMaxK + 1] = {};
+    int64_t qlen[32];
+    for (int64_t x = 0; x < qn; x++) {
+        const int64_t i = nq * x / qn;
+        q[x] = signature(bq + oq[i], qlen[x] = oq[i + 1] - oq[i]);
+    }
+    int pass[kSigMaxK + 1] = {}, near[kSigMaxK + 1] = {};
     for (int64_t y = 0; y < cn; y++) {
-        const Sig g = signature(bc + oc[nc * y / cn], oc[nc * y / cn + 1] - oc[nc * y / cn]);
+        const int64_t i = nc * y / cn, len = oc[i + 1] - oc[i];
+        const Sig g = signature(bc + oc[i], len);
         for (int64_t x = 0; x < qn; x++) {
             int diff = 0;
-            for (int w = 0; w < kSigWords / 2; w++) diff += __builtin_popcountll(q[x].w[w] ^ g.w[w]);
-            const int k = (diff + 7) / 8;
-            if (k <= kSigMaxK) count[k]++;
+            for (int w = 0; w < 4; w++) diff += __builtin_popcountll(q[x].w[w] ^ g.w[w]);
+            const int64_t k = (diff + 7) / 8, both = std::max(k, std::abs(qlen[x] - len));
+            if (k <= kSigMaxK) pass[k]++;
+            if (both <= kSigMaxK) near[both]++;
         }
     }
-    int sum = 0;
+    int sum = 0, sum_near = 0;
     for (int k = 0; k <= kSigMaxK; k++) {
-        sum += count[k];
-        s->gram_pass[k] = (float)sum / (float)(qn * cn);
+        s->gram_pass[k] = (float)(sum += pass[k]) / (float)(qn * cn);
+        s->gram_near[k] = (float)(sum_near += near[k]) / (float)(qn * cn);
     }
 }
-
 
 // One-call cdist with host results: queries in chunks of rows; the rows of
 // chunk i go back (stream `down`) while chunk i+1 computes.
@@ -1996,11 +2004,11 @@ static FilterPlan filter_plan(const blg_ctx *c, const blg_search *s, const SurvC
     f.nq = (int)nq;
     f.folded = pass_folded <= pass + 1e-7 * pairs;
     f.filter_us = 6.0 + std::ceil(tiles / c->sms) * (f.folded ? 0.75 : 1.15);
-    const double share = s->gram_pass[k], related = share * (double)nq * (double)s->nc;
+    const double all = (double)nq * (double)s->nc, share = s->gram_pass[k];
     const bool brief = s->c.d.bytes <= 72 * s->nc;
-    const double room = std::min(pairs / (brief ? 4.0 : 16.0), (brief ? 1.25 : 0.75) * (double)c->pl_cap);
     f.pays = pairs >= 1800.0 * tiles && pairs >= kFltMinPairs && pass <= std::min((double)c->pl_cap / 8.0, pairs / 32.0) &&
-             (related <= room || share >= 0.9);
+             ((share * all <= (brief ? 1.25 : 0.75) * (double)c->pl_cap && s->gram_near[k] * all <= pairs / (brief ? 4.0 : 16.0)) ||
+              share >= 0.9);
     return f;
 }
 
@@ -3768,12 +3776,12 @@ int blg_cdist_matches(blg_ctx *c, const uint8_t *bq, const int64_t *oq, int64_t 
     const unsigned need = surv ? NEED_SORTED : NEED_TT;
     int rc = search_upload_queries(c, bq, oq, nq, &s, need);
     if (!rc) rc = search_upload_choices(c, bc, oc, nc, &s, need);
-    if (!rc) sample_grams(bq, oq, nq, bc, oc, nc, &s);
     // the survivor kernel's result list, where the run qualifies
     int64_t total = 0;
     bool listed = false;
     if (!rc && surv && max_dist <= 31) {
         rc = search_build_classes(c, oq, 0, nq, &s);
+        if (!rc && filter_plan(c, &s, seq_classes(&s), max_dist).pays) sample_grams(bq, oq, nq, bc, oc, nc, &s);
         if (!rc) rc = search_matches_list(c, &s, max_dist, nullptr, out, capacity, &total, &listed);
     }
     // else query rows in chunks whose dense scratch stays within the budget

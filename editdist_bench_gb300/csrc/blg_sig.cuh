@@ -19,9 +19,10 @@ constexpr int kSigWords = 8;                     // 32 bytes per string
 constexpr int kSigBins = 248;                    // bits 6 and 7 of the last word's bytes stay 0
 constexpr int kSigMaxK = 15;                     // largest k whose e4m3 is exact as it stands
 
-// bit position (word << 5 | bit) of a 4-gram g (its bytes in order, first highest)
+// bin of a 4-gram g (its bytes in order, first highest), and its bit's position (word << 5 | bit)
+BLG_HD uint32_t sig_bin(uint32_t g) { return (((g * 0x9E3779B1u) >> 16) * (uint32_t)kSigBins) >> 16; }
 BLG_HD uint32_t sig_bit(uint32_t g) {
-    const uint32_t bin = (((g * 0x9E3779B1u) >> 16) * (uint32_t)kSigBins) >> 16;
+    const uint32_t bin = sig_bin(g);
     if (bin < 224u) return bin;
     const uint32_t r = bin - 224u;               // 24 bins: six low bits of each byte of the last word
     return 224u + 8u * (r / 6u) + r % 6u;

@@ -5,7 +5,8 @@ import numpy as np
 import pytest
 
 import oracle
-from editdist_bench_gb300 import workloads as W
+from editdist_bench_gb300 import _lib, workloads as W
+from test_gpu_prefix import _labels
 from test_search_filter import TEXT, _run, _sets
 
 pytestmark = pytest.mark.gpu
@@ -72,3 +73,16 @@ def test_batch_unit_sizes(gpu, nq, nc):
     for rep in range(2):
         for got, (q, c, k, dt) in zip([o.get() for o in b.run()], probs):
             np.testing.assert_array_equal(got, oracle.saturate(oracle.cross(q, c, k, threads=16), dt))
+
+
+def test_filter_counts_passers_within_the_window(gpu):
+    """Short strings pass the 4-gram test whatever their lengths' difference; only those
+    within it are solved."""
+    rng = np.random.default_rng(5)
+    q, c = (W.random_strings(rng, rng.integers(38, 174, n)) for n in (379, 123334))
+    got = []
+    labels = _labels(_lib.context(), lambda: got.append(gpu.cdist_matches_packed(q, c, 6)))
+    assert "filter_pairs" in labels, labels
+    wi, wj = np.nonzero(oracle.cross(q, c, 6, threads=8) <= 6)
+    np.testing.assert_array_equal(got[0][0], wi)
+    np.testing.assert_array_equal(got[0][1], wj)
