@@ -231,8 +231,9 @@ struct blg_search {
     double warp_len = 0.0;            // mean of the longest of 32 neighbours
     int gram_sym = 256;              // the queries' bytes, as that many equally frequent ones (filter_plan)
     // by k: share of a sample's pairs whose 4-grams allow it, and of those the ones whose
-    // lengths do (sample_grams)
+    // lengths do (sample_grams; sampled: there was one)
     float gram_pass[kSigMaxK + 1] = {}, gram_near[kSigMaxK + 1] = {};
+    bool sampled = false;
     // exact runs, bit-sliced over the queries (k_search_bits): the distinct
     // bytes of the queries (nsym 0: not counted, or too many) and, per class set, the
     // sequential queries by length
@@ -1574,11 +1575,13 @@ static int search_upload_queries(blg_ctx *c, const uint8_t *bq, const int64_t *o
 
 // Of 32 queries x 64 choices spread over the sets, the share whose signatures differ
 // by at most 8 k, and whose lengths by at most k beside that, for every k of the filter
-// (filter_plan). The first 512 bytes of a string stand for it. Host work
+// (filter_plan, search_small). The first 512 bytes of a string stand for it. Host work
 // beside the choices' upload. (The bins as they are hashed: sig_bit's places give the same counts.)
+constexpr double kSampleMinPairs = 5e5;
+
 static void sample_grams(const uint8_t *bq, const int64_t *oq, int64_t nq, const uint8_t *bc, const int64_t *oc, int64_t nc,
                          blg_search *s) {
-    if (!s->csig || (double)nq * (double)nc < 1.5 * kFltMinPairs) return;   // (search_small takes what is smaller)
+    if (!s->csig || (double)nq * (double)nc < kSampleMinPairs) return;
     struct Sig {
         uint64_t w[4] = {};
     };
@@ -1617,6 +1620,7 @@ static void sample_grams(const uint8_t *bq, const int64_t *oq, int64_t nq, const
         s->gram_pass[k] = (float)(sum += pass[k]) / (float)(qn * cn);
         s->gram_near[k] = (float)(sum_near += near[k]) / (float)(qn * cn);
     }
+    s->sampled = true;
 }
 
 // One-call cdist with host results: queries in chunks of rows; the rows of
@@ -1766,9 +1770,17 @@ static int survivor_job_size(blg_ctx *c, const Window &w, int k) {
 // equal and a sixteenth of the pairs related (reads of 64 of 16 families), 64 x 40000, 64
 // x 20000: k = 1 19 / 38, 15 / 34; k = 2 53 / 47, 34 / 41; k = 3 107 / 54, 60 / 46 (16 x
 // 60000: 54 / 45), texts at k = 8 104 / 85, at 12 114 / 120 (64 x 40000 218 / 204).
+// Unrelated strings leave the band after some 2 k columns: where none of a sample
+// passes the test hardly a warp walks, and where an eighth of the window passes and
+// next to none at half of k there is nothing to pack (132 x 17251 DNA of 42, k = 6: 77 /
+// 132; 154 x 10409 of 106 to 201, k = 8: 43 / 66).
 static bool search_small(const blg_search *s, const Window &w, double pairs, int k) {
     const bool short_choices = s->min_len + s->n_len - 1 <= 64;
-    return pairs <= (short_choices ? 4e6 : 1.7e6) && w.columns <= (k <= 1 ? 2.4e8 : k == 2 ? 7e7 : k < 12 ? 4e7 : 1.1e8);
+    if (pairs > (short_choices ? 4e6 : 1.7e6)) return false;
+    if (w.columns <= (k <= 1 ? 2.4e8 : k == 2 ? 7e7 : k < 12 ? 4e7 : 1.1e8)) return true;
+    if (!s->sampled || k > kSigMaxK) return false;
+    const double near = s->gram_near[k];
+    return near < 1.0 / 1024.0 || (8.0 * near * pairs >= (double)w.pairs && 64.0 * s->gram_near[k / 2] <= near);
 }
 
 // The sequential (not lane-spread) query classes of a search, for the

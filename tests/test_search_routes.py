@@ -75,6 +75,18 @@ def test_batch_unit_sizes(gpu, nq, nc):
             np.testing.assert_array_equal(got, oracle.saturate(oracle.cross(q, c, k, threads=16), dt))
 
 
+# unrelated strings: none passes the 4-gram test, or so many that nothing is left to pack
+@pytest.mark.parametrize("nq,nc,lo,hi,k,small", [(40, 25001, 64, 64, 3, True), (132, 17251, 42, 42, 6, True),
+                                                 (154, 10409, 106, 201, 8, True), (40, 25001, 64, 64, 6, False)])
+def test_small_search_of_unrelated_strings(gpu, nq, nc, lo, hi, k, small):
+    rng = np.random.default_rng(nq)
+    q, c = (W.random_strings(rng, rng.integers(lo, hi + 1, n)) for n in (nq, nc))
+    s = gpu.SearchBatch(q, c)
+    got, labels = _run(gpu, s, s.alloc("uint8"), k)
+    assert ("search_small" in labels) == small, labels
+    np.testing.assert_array_equal(got, oracle.saturate(oracle.cross(q, c, k, threads=8), "uint8"))
+
+
 def test_filter_counts_passers_within_the_window(gpu):
     """Short strings pass the 4-gram test whatever their lengths' difference; only those
     within it are solved."""
