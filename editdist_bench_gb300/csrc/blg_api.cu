@@ -1770,17 +1770,20 @@ static int survivor_job_size(blg_ctx *c, const Window &w, int k) {
 // equal and a sixteenth of the pairs related (reads of 64 of 16 families), 64 x 40000, 64
 // x 20000: k = 1 19 / 38, 15 / 34; k = 2 53 / 47, 34 / 41; k = 3 107 / 54, 60 / 46 (16 x
 // 60000: 54 / 45), texts at k = 8 104 / 85, at 12 114 / 120 (64 x 40000 218 / 204).
-// Unrelated strings leave the band after some 2 k columns: where none of a sample
-// passes the test hardly a warp walks, and where an eighth of the window passes and
-// next to none at half of k there is nothing to pack (132 x 17251 DNA of 42, k = 6: 77 /
-// 132; 154 x 10409 of 106 to 201, k = 8: 43 / 66).
+// Unrelated strings leave the band after some 2 k columns: where next to none of a sample
+// passes the test hardly a warp walks (231 x 15976 texts of 34, k = 5: 66 / 100; at k = 2
+// a 500th of related ones is enough for 53 / 47), and where an eighth of the window
+// passes and next to none at half of k there is nothing to pack (132 x 17251 DNA of 42,
+// k = 6: 77 / 132; 154 x 10409 of 106 to 201, k = 8: 43 / 66; 179 x 17754 texts of 85, k =
+// 12: 103 / 140; 153 x 15607 DNA of 73 to 185, k = 12: 50 / 77).
 static bool search_small(const blg_search *s, const Window &w, double pairs, int k) {
-    const bool short_choices = s->min_len + s->n_len - 1 <= 64;
-    if (pairs > (short_choices ? 4e6 : 1.7e6)) return false;
-    if (w.columns <= (k <= 1 ? 2.4e8 : k == 2 ? 7e7 : k < 12 ? 4e7 : 1.1e8)) return true;
+    const double room = s->min_len + s->n_len - 1 <= 64 ? 4e6 : 1.7e6;
+    if (pairs > 4e6) return false;
+    if (pairs <= room && w.columns <= (k <= 1 ? 2.4e8 : k == 2 ? 7e7 : k < 12 ? 4e7 : 1.1e8)) return true;
     if (!s->sampled || k > kSigMaxK) return false;
     const double near = s->gram_near[k];
-    return near < 1.0 / 1024.0 || (8.0 * near * pairs >= (double)w.pairs && 64.0 * s->gram_near[k / 2] <= near);
+    if (8.0 * near * pairs >= (double)w.pairs && 64.0 * s->gram_near[k / 2] <= near) return true;
+    return pairs <= room && near < (k < 3 ? 1.0 / 1024.0 : 1.0 / 256.0);
 }
 
 // The sequential (not lane-spread) query classes of a search, for the

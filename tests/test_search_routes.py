@@ -98,3 +98,14 @@ def test_filter_counts_passers_within_the_window(gpu):
     wi, wj = np.nonzero(oracle.cross(q, c, 6, threads=8) <= 6)
     np.testing.assert_array_equal(got[0][0], wi)
     np.testing.assert_array_equal(got[0][1], wj)
+
+
+# a few of the pairs pass, or most of a window that holds all of them: texts
+@pytest.mark.parametrize("nq,nc,length,k", [(231, 15976, 34, 5), (179, 17754, 85, 12)])
+def test_small_search_of_unrelated_texts(gpu, nq, nc, length, k):
+    rng = np.random.default_rng(k)
+    q, c = (W.random_strings(rng, np.full(n, length), TEXT) for n in (nq, nc))
+    s = gpu.SearchBatch(q, c)
+    got, labels = _run(gpu, s, s.alloc("uint8"), k)
+    assert "search_small" in labels, labels
+    np.testing.assert_array_equal(got, oracle.saturate(oracle.cross(q, c, k, threads=8), "uint8"))
